@@ -173,6 +173,14 @@ int inlm_debug_live_allocations(int64_t* n);
  * records the timeout in the handle's error word and returns, and this call
  * returns INLM_ERR_TIMEOUT as a filter call would. The handle stays usable. */
 int inlm_debug_wait_expiry(inlm_denoiser* d, int64_t cycles);
+/* Test hooks of the paired-offset FP32 form. inlm_debug_pair_workspace bounds
+ * the handle's workspace to `bytes` (0: the default), so that small volumes are
+ * cut into blocks and z chunks as large ones are; INLM_ERR_UNSUPPORTED where
+ * the form does not run. inlm_debug_weight_mismatches compares, on the current
+ * device, the form's weight step with the other kernels' for every float x in
+ * [-3.6, -0] and stores how many differ. */
+int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes);
+int inlm_debug_weight_mismatches(int64_t* n);
 
 /* Number of kernels this handle has launched since creation. */
 int inlm_kernel_launches(inlm_denoiser* d, uint64_t* count);

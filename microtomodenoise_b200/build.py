@@ -37,8 +37,11 @@ LIB_SOURCES = [
     "filter_kernels.cu",
     "filter_column.cu",
     "filter_fast.cu",
+    "filter_pair.cu",
+    "filter_pair_weight.cu",
     "noise_kernels.cu",
     "api.cu",
+    "api_pair.cu",
     "proposal.cu",
     "proposal_tc.cu",
     "api_proposal.cu",

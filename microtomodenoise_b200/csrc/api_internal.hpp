@@ -17,6 +17,7 @@
 #include "../../include/inlm.h"
 #include "filter_fast.cuh"
 #include "filter_kernels.cuh"
+#include "filter_pair.cuh"
 #include "geometry.hpp"
 #include "proposal.cuh"
 
@@ -143,6 +144,25 @@ struct ProposalRun {
     inlm::DevBuf a1, a2, a3, a4, bitmap, pmass, counters, scale, plan_start, plan_off, mass_sum;
 };
 
+// Paired-offset FP32 form (api_pair.cu): its plan and workspace.
+struct PairRun {
+    bool active = false;   // filters of this handle run the paired form
+    bool planned = false;  // blocks chosen
+    int bx = 0, by = 0;    // voxels per block in x and y
+    int tz = 0;            // deepest tile that fits in shared memory
+    int chunk = 0;         // planes per pair of launches
+    int warps = 0;         // warps per CTA
+    inlm::PairArgs args{};
+    inlm::PairMaps maps{};
+    int sms = 0;
+    inlm::DevBuf offsets, z_start;
+    size_t limit = 0;       // bound on the workspace set by a test (0: none)
+    size_t bytes = 0;       // workspace the plan needs
+    void* dist = nullptr;   // borrowed workspace (pair_idle hands it back)
+    size_t dist_bytes = 0;
+    bool user = false;      // counted among the pool's users
+};
+
 struct inlm_denoiser {
     int shape[3] = {0, 0, 0};
     inlm_params p;
@@ -195,6 +215,7 @@ struct inlm_denoiser {
     inlm::TileConfig tcfg{};
     inlm::TileArgs targs{};
     inlm::GenericArgs gargs{};
+    PairRun pair;
     CUtensorMap tm_prev{}, tm_raw{};
     int last_iter = 0;
     bool sigma_set = false;
@@ -212,6 +233,20 @@ int launch_filter(inlm_denoiser* d);
 int check_device_error(inlm_denoiser* d);
 int tile_config_try(inlm_denoiser* d, int tz, bool raw_smem, bool* ok, bool ws = false);
 int upload_sigma_device(inlm_denoiser* d);
+// TMA map of a float array: rank (3 or 4) extents, pitches of axes 1.. in
+// elements, box.
+int encode_map_f32(CUtensorMap* tm, const void* base, int rank, const long long* dims, const long long* pitch,
+                   const int* box);
+// Paired-offset form: decides whether it covers the handle (after the tile
+// configuration), plans and borrows a workspace, runs one filter pass, hands the
+// workspace back (the handle's work on the GPU has ended), releases everything.
+// pair_trim frees the workspace no handle has borrowed (true if there was one).
+int pair_configure(inlm_denoiser* d);
+int pair_prepare(inlm_denoiser* d, bool* ready);
+int pair_filter(inlm_denoiser* d);
+void pair_idle(inlm_denoiser* d);
+void pair_release(inlm_denoiser* d);
+bool pair_trim(int device);
 int pad_into(inlm_denoiser* d, const float* src, float* dst);
 int pad_into_half(inlm_denoiser* d, const float* src, void* dst);
 // Noise estimate of a device volume into d_dst (nz floats, device); host_copy

@@ -1,0 +1,362 @@
+// Host side of the paired-offset FP32 form (filter_pair.cu): when it applies,
+// the workspace and how a volume is cut into blocks and z chunks that fit it.
+#include <mutex>
+
+#include "api_internal.hpp"
+#include "common.cuh"
+
+using namespace inlm;
+
+namespace {
+
+// A workspace takes at most an eighth of the device's memory, and half of what
+// is free when a handle plans its passes. A deeper z chunk means fewer launches
+// with a partly filled last wave: 256^3, patch radius 1, search radius 10 takes
+// 95 ms with an eighth and 101 ms with a sixteenth.
+constexpr int kWorkspaceShare = 8;
+
+// Workspaces are not the handles': a call borrows one and hands it back when
+// its work on the GPU has ended, so handles that take turns share one buffer.
+// Per device the pool keeps at most one idle buffer, and none once the last
+// handle that borrowed is gone.
+struct Pool {
+    void* idle = nullptr;
+    size_t idle_bytes = 0;
+    int users = 0;
+};
+constexpr int kMaxDevices = 64;
+Pool g_pool[kMaxDevices];
+std::recursive_mutex g_pool_mutex;  // device_malloc may call pair_trim under it
+
+cudaError_t borrow(int device, size_t bytes, void** p, size_t* got) {
+    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
+    Pool& pool = g_pool[device];
+    if (pool.idle && pool.idle_bytes < bytes) {
+        device_free(pool.idle);
+        pool.idle = nullptr;
+    }
+    if (pool.idle) {
+        *p = pool.idle;
+        *got = pool.idle_bytes;
+        pool.idle = nullptr;
+        return cudaSuccess;
+    }
+    const cudaError_t e = device_malloc(p, bytes);
+    if (e == cudaSuccess) *got = bytes;
+    return e;
+}
+
+void hand_back(int device, void* p, size_t bytes) {
+    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
+    Pool& pool = g_pool[device];
+    if (pool.users > 0 && (!pool.idle || pool.idle_bytes < bytes)) {
+        std::swap(p, pool.idle);
+        pool.idle_bytes = bytes;
+    }
+    device_free(p);
+}
+
+void count_user(int device, int change) {
+    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
+    Pool& pool = g_pool[device];
+    pool.users += change;
+    if (pool.users == 0) {
+        device_free(pool.idle);
+        pool.idle = nullptr;
+    }
+}
+
+size_t idle_bytes(int device) {
+    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
+    return g_pool[device].idle ? g_pool[device].idle_bytes : 0;
+}
+
+int round_up(int v, int m) { return (v + m - 1) / m * m; }
+
+// CTAs that share one tile's offsets: as many as leave the least of the last
+// wave empty (one CTA runs per SM), each costing another load of the tile's
+// box (about a fiftieth of a tile's work), and at most one per round of warps.
+int offset_splits(int tiles, int sms, int most) {
+    int best = 1;
+    double best_cost = 0;
+    for (int n = 1; n <= std::max(1, std::min(most, 64)); n++) {
+        const double cost = (double)((tiles * (long long)n + sms - 1) / sms) / n * (1.0 + 0.02 * n);
+        if (n == 1 || cost < best_cost) {
+            best = n;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+}  // namespace
+
+// Whether the paired form covers the handle's configuration: an instantiated
+// patch shape whose taps the tile kernel checked, weights that depend on
+// |x|, |y|, |z| alone, and offsets in central symmetry with the first half
+// at z <= 0 (the reference's z-major order always is).
+int inlm::pair_configure(inlm_denoiser* d) {
+    PairRun& r = d->pair;
+    r.active = false;
+    const Geometry& g = d->geo;
+    const int* pr = g.patch_radius;
+    const int S = (int)g.search.size();
+    if (!d->use_tile || d->device >= kMaxDevices || S < 2 || S % 2 || !pair_kernel_available(pr[0], pr[1], pr[2]))
+        return INLM_OK;
+    if (!pair_weights_symmetric(pr[0], pr[1], pr[2], d->targs.w)) return INLM_OK;
+    for (int s = 0; s < S / 2; s++) {
+        const Offset3 &o = g.search[s], &m = g.search[S - 1 - s];
+        if (o.x != -m.x || o.y != -m.y || o.z != -m.z || o.z > 0) return INLM_OK;
+    }
+    for (int s = 1; s < S; s++)
+        if (g.search[s].z < g.search[s - 1].z) return INLM_OK;
+    PairArgs& a = r.args;
+    a = PairArgs{};
+    a.nx = d->shape[0];
+    a.ny = d->shape[1];
+    a.nz = d->shape[2];
+    a.px = g.pad[0];
+    a.py = g.pad[1];
+    a.pz = g.pad[2];
+    a.sxr = g.search_radius[0];
+    a.syr = g.search_radius[1];
+    a.szc = std::min(d->p.nslices / 2, g.search_radius[2]);
+    a.S = S;
+    a.H = S / 2;
+    a.pbx = pair_box_pitch(a.px);
+    if (a.pbx == 0) return INLM_OK;
+    a.pby = 8 + 2 * a.py;
+    for (int t = 0; t < (int)g.taps.size(); t++) a.w[t] = g.weights[t];
+    // the deepest tile whose box fits beside the warps' buffers
+    int smem_max = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
+    a.tz = 0;
+    for (int tz = 24; tz >= 4 && a.tz == 0; tz--) {
+        a.pbz = tz + 2 * pr[2] + a.szc;
+        if (pair_smem_bytes(pr[0], pr[2], a) <= (size_t)smem_max) a.tz = tz;
+    }
+    if (a.tz == 0 || a.pbx > 256 || a.pby > 256 || a.pbz > 256) return INLM_OK;
+    r.tz = a.tz;
+    r.planned = false;
+    r.active = true;
+    return INLM_OK;
+}
+
+// Cuts the volume into blocks (whole rows and columns where they fit) and each
+// block into z chunks, so that one chunk's distances and the search halo fit
+// the workspace; builds the offset table. Sets r.active = false where not
+// even the smallest block fits.
+static int pair_plan(inlm_denoiser* d) {
+    PairRun& r = d->pair;
+    PairArgs& a = r.args;
+    const Geometry& g = d->geo;
+    size_t free_b = 0, total_b = 0;
+    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    size_t budget = std::min(total_b / kWorkspaceShare, (free_b + idle_bytes(d->device)) / 2);
+    if (r.limit > 0) budget = std::min(budget, r.limit);
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
+    const int depth = a.nz + a.szc;  // planes whose distances are read
+    const int tz_most = r.tz;
+    double best = 0;
+    for (int nby = 1; nby <= 32; nby++)
+        for (int nbx = 1; nbx <= 32; nbx++) {
+            const int bx = round_up((a.nx + nbx - 1) / nbx, 32), by = round_up((a.ny + nby - 1) / nby, 8);
+            if ((nbx > 1 && bx * (nbx - 1) >= a.nx) || (nby > 1 && by * (nby - 1) >= a.ny)) continue;
+            const int tiles_x = (round_up(a.sxr, 8) + std::min(bx, a.nx) + a.sxr + 31) / 32;
+            const int tiles_y = (2 * a.syr + std::min(by, a.ny) + 7) / 8;
+            const size_t plane = (size_t)tiles_x * 32 * tiles_y * 8 * a.H * 4;
+            const int ring_max = (int)std::min<size_t>(budget / plane, 1 << 20);
+            int chunk = depth, ring = depth, tz = tz_most;
+            if (ring > ring_max) {
+                // as few chunks of whole tiles as fit, or tiles as deep as fit
+                tz = std::min(tz, ring_max - a.szc);
+                if (tz < 4) continue;
+                chunk = (ring_max - a.szc) / tz * tz;
+                const int n = (depth + chunk - 1) / chunk;
+                chunk = round_up((depth + n - 1) / n, tz);
+                ring = chunk + a.szc;
+            }
+            const int tiles_z = (chunk + tz - 1) / tz, n_chunks = (depth + chunk - 1) / chunk;
+            // tiles of all launches, and a third of a wave of tiles lost at
+            // the end of each
+            const double tiles = (double)tiles_x * tiles_y * tiles_z;
+            // (a tile of tz planes walks tz + 2 RZ)
+            const double cost = (tiles / sms + 0.3) * (tz + 2 * g.patch_radius[2]) * n_chunks * nbx * nby;
+            if (best == 0 || cost < best) {
+                best = cost;
+                r.bx = bx;
+                r.by = by;
+                r.chunk = chunk;
+                a.tz = tz;
+                a.pbz = tz + 2 * g.patch_radius[2] + a.szc;
+                a.tiles_x = tiles_x;
+                a.tiles_y = tiles_y;
+                a.ex = tiles_x * 32;
+                a.ey = tiles_y * 8;
+                a.ring = ring;
+            }
+        }
+    if (best == 0) {
+        r.active = false;
+        return INLM_OK;
+    }
+    const int S = a.S;
+    std::vector<PairOffset> t(S);
+    for (int s = 0; s < S; s++) {
+        const Offset3& o = g.search[s];
+        t[s].x = o.x;
+        t[s].y = o.y;
+        t[s].z = o.z;
+        t[s].prev = (o.z * a.pby + o.y) * a.pbx + o.x;
+    }
+    std::vector<int> zs(2 * a.szc + 2, S);  // first offset of every z
+    for (int s = S - 1; s >= 0; s--) zs[g.search[s].z + a.szc] = s;
+    for (int i = 2 * a.szc; i >= 0; i--) zs[i] = std::min(zs[i], zs[i + 1]);
+    r.bytes = (size_t)a.H * a.ring * a.ex * a.ey * 4;
+    CUDA_TRY(r.offsets.ensure(S * sizeof(PairOffset)));
+    CUDA_TRY(r.z_start.ensure(zs.size() * sizeof(int)));
+    CUDA_TRY(cudaMemcpyAsync(r.offsets.p, t.data(), S * sizeof(PairOffset), cudaMemcpyHostToDevice, d->stream));
+    CUDA_TRY(cudaMemcpyAsync(r.z_start.p, zs.data(), zs.size() * sizeof(int), cudaMemcpyHostToDevice, d->stream));
+    CUDA_TRY(cudaStreamSynchronize(d->stream));  // the host vectors go out of scope
+    a.offsets = r.offsets.as<PairOffset>();
+    a.z_start = r.z_start.as<int>();
+    a.neg0 = -0.0f;
+    a.raw_pad = d->d_raw_pad;
+    a.gpitch_y = d->pitch_y;
+    a.gpitch_z = d->pitch_z;
+    a.out = d->d_next;
+    a.mult = d->d_mult;
+    a.err = d->d_err;
+    r.sms = sms;
+    r.warps = pair_kernel_warps(g.patch_radius[0]);
+    r.planned = true;
+    return INLM_OK;
+}
+
+// Borrows a workspace for the handle's next passes; *ok = false where there is
+// no room for one.
+static int pair_borrow(inlm_denoiser* d, bool* ok) {
+    PairRun& r = d->pair;
+    PairArgs& a = r.args;
+    *ok = true;
+    if (r.dist) return INLM_OK;
+    if (!r.user) {
+        count_user(d->device, 1);
+        r.user = true;
+    }
+    if (borrow(d->device, r.bytes, &r.dist, &r.dist_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        r.dist = nullptr;
+        *ok = false;
+        return INLM_OK;
+    }
+    if (a.dist == r.dist) return INLM_OK;  // the tensor maps are this buffer's
+    a.dist = nullptr;
+    const long long pad_dims[3] = {d->nxp, d->nyp, d->nzp}, pad_pitch[2] = {d->pitch_y, d->pitch_z};
+    const int box[3] = {a.pbx, a.pby, a.pbz};
+    int rc = encode_map_f32(&r.maps.prev, d->d_prev_pad, 3, pad_dims, pad_pitch, box);
+    const int obox[4] = {32, 8, 1, 1};
+    const long long dims[4] = {a.ex, a.ey, a.ring, a.H};
+    const long long pitch[3] = {a.ex, (long long)a.ex * a.ey, (long long)a.ex * a.ey * a.ring};
+    if (rc == INLM_OK) rc = encode_map_f32(&r.maps.out, r.dist, 4, dims, pitch, obox);
+    for (int i = 0; i < 2 && rc == INLM_OK; i++) {
+        const int dbox[4] = {kPairDistBox, pair_weight_rows(i), 1, 1};
+        const int rbox[3] = {a.pbx, pair_weight_rows(i) + 2 * a.syr, 1};
+        rc = encode_map_f32(&r.maps.dist[i], r.dist, 4, dims, pitch, dbox);
+        if (rc == INLM_OK) rc = encode_map_f32(&r.maps.raw[i], d->d_raw_pad, 3, pad_dims, pad_pitch, rbox);
+    }
+    if (rc) return rc;
+    a.dist = static_cast<float*>(r.dist);
+    return INLM_OK;
+}
+
+// Plans the handle's passes and borrows their workspace; *ready = false when the
+// form does not run here.
+int inlm::pair_prepare(inlm_denoiser* d, bool* ready) {
+    PairRun& r = d->pair;
+    *ready = false;
+    if (r.active && !r.planned) {
+        const int rc = pair_plan(d);
+        if (rc) return rc;
+    }
+    return r.active ? pair_borrow(d, ready) : INLM_OK;
+}
+
+// Enqueues one filter pass.
+int inlm::pair_filter(inlm_denoiser* d) {
+    const PairRun& r = d->pair;
+    const int* pr = d->geo.patch_radius;
+    const bool fused = d->p.precision == INLM_PRECISION_F32_FMA;
+    PairArgs a = r.args;
+    const int depth = a.nz + a.szc;
+    for (int y0 = 0; y0 < a.ny; y0 += r.by)
+        for (int x0 = 0; x0 < a.nx; x0 += r.bx) {
+            a.x0 = x0;
+            a.x1 = std::min(a.nx, x0 + r.bx);
+            a.y0 = y0;
+            a.y1 = std::min(a.ny, y0 + r.by);
+            a.xs = x0 - round_up(a.sxr, 8);
+            a.ys = y0 - a.syr;
+            a.tiles_x = (a.x1 + a.sxr - a.xs + 31) / 32;
+            a.tiles_y = (a.y1 + a.syr - a.ys + 7) / 8;
+            for (int z = 0; z < depth; z += r.chunk) {
+                const int z1 = std::min(depth, z + r.chunk);
+                a.tiles_z = (z1 - z + a.tz - 1) / a.tz;
+                a.splits = offset_splits(a.tiles_x * a.tiles_y * a.tiles_z, r.sms, (a.H + r.warps - 1) / r.warps);
+                CUDA_TRY(launch_pair_dist(pr[0], pr[1], pr[2], fused, r.maps, a, z, d->stream));
+                CUDA_TRY(launch_pair_weights(fused, r.maps, a, std::max(0, z - a.szc), std::min(a.nz, z1 - a.szc), r.sms,
+                                             d->stream));
+                d->launches += 2;
+            }
+        }
+    return INLM_OK;
+}
+
+bool inlm::pair_trim(int device) {
+    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
+    if (device < 0 || device >= kMaxDevices || !g_pool[device].idle) return false;
+    device_free(g_pool[device].idle);
+    g_pool[device].idle = nullptr;
+    return true;
+}
+
+void inlm::pair_idle(inlm_denoiser* d) {
+    PairRun& r = d->pair;
+    if (r.dist) hand_back(d->device, r.dist, r.dist_bytes);
+    r.dist = nullptr;
+}
+
+void inlm::pair_release(inlm_denoiser* d) {
+    PairRun& r = d->pair;
+    pair_idle(d);
+    if (r.user) count_user(d->device, -1);
+    r.user = false;
+    r.offsets.release();
+    r.z_start.release();
+    r.planned = false;
+}
+
+extern "C" int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes) {
+    if (!d || bytes < 0) return fail(INLM_ERR_ARG, "bad argument");
+    if (!d->pair.active) return fail(INLM_ERR_UNSUPPORTED, "the paired form does not run on this handle");
+    CUDA_TRY(cudaSetDevice(d->device));
+    CUDA_TRY(cudaStreamSynchronize(d->stream));
+    pair_release(d);
+    d->pair.limit = (size_t)bytes;
+    return INLM_OK;
+}
+
+extern "C" int inlm_debug_weight_mismatches(int64_t* n) {
+    if (!n) return fail(INLM_ERR_ARG, "null argument");
+    unsigned long long* dn = nullptr;
+    CUDA_TRY(dalloc(&dn, 1));
+    unsigned long long h = 0;
+    cudaError_t e = cudaMemset(dn, 0, sizeof h);
+    if (e == cudaSuccess) e = launch_weight_mismatches(dn, -0.0f, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(&h, dn, sizeof h, cudaMemcpyDeviceToHost);
+    device_free(dn);
+    CUDA_TRY(e);
+    *n = (int64_t)h;
+    return INLM_OK;
+}

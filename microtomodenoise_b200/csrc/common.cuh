@@ -80,6 +80,30 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tm, in
         : "memory");
 }
 
+// 4D tiled TMA load (no multicast); the same rule for x.
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, int x, int y, int z, int w,
+                                            uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// 4D tiled TMA store of a shared-memory tile as a bulk group of its own (the
+// issuing thread's); the writes to src must be fenced for the async proxy.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* tm, const void* src, int x, int y, int z, int w) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
+            reinterpret_cast<uint64_t>(tm)),
+        "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(src))
+        : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// The thread's stores have read their source / have completed.
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* tm) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
 }

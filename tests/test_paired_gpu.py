@@ -1,0 +1,147 @@
+"""The paired-offset FP32 form: distances of half of the search offsets, each
+used for both offsets of a pair. Bit-exact to the oracle at the edges of its
+tiles, z chunks, blocks and row forms, and where it has no workspace."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from microtomodenoise_b200 import DenoiseParameters, IterativeNLM_GPU, _lib, synth
+from oracle.oracle import FilterParams
+
+MB = 1 << 20
+
+
+def _run(raw, pr, sr, sig, limit=0, nslices=11, precision="f32", form=None):
+    g = IterativeNLM_GPU()
+    g.configure_device(raw.shape, DenoiseParameters(radius_patchspace=pr, radius_searchspace=sr, nslices=nslices,
+                                                    precision=precision))
+    if form:
+        g.select_tile_form(form)
+    else:
+        assert "paired" in g.describe(), g.describe()
+        _lib.check(_lib.load().inlm_debug_pair_workspace(g._h, limit), "pair_workspace")
+    outs = []
+    for it in range(len(sig)):
+        g.set_sigma(sig[it])
+        g.Run_GaussianNoise(it + 1, raw if it == 0 else None)
+        outs.append(g.get_result())
+    desc = g.describe()
+    g.free_device()
+    return np.stack(outs), desc
+
+
+def _sigmas(nz):
+    return np.stack([np.full(nz, 0.07, np.float32), np.linspace(0.03, 0.08, nz, dtype=np.float32)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,pr,sr,limit", [
+    ((9, 19, 41), (2, 2, 2), (3, 4, 2), 0),           # one chunk, uneven search radii
+    ((5, 7, 9), (1, 1, 1), (2, 2, 2), 0),             # smaller than a tile in every axis
+    ((3, 40, 40), (1, 1, 1), (4, 4, 4), 0),           # fewer planes than the z halo
+    ((61, 23, 70), (1, 1, 1), (4, 4, 4), 24 * MB),    # z chunks, ring wraps
+    ((43, 40, 100), (2, 2, 2), (3, 3, 3), 4 * MB),    # blocks in x and y too
+    ((34, 17, 45), (3, 3, 3), (3, 3, 3), 4 * MB),     # direct columns, z chunks
+    ((13, 9, 70), (2, 2, 1), (5, 5, 5), 0),
+    ((16, 24, 40), (1, 1, 2), (6, 6, 6), 0),
+    ((12, 30, 33), (1, 1, 3), (3, 3, 3), 0),
+    ((14, 18, 33), (3, 3, 1), (2, 2, 2), 0),
+    ((11, 16, 32), (3, 3, 2), (4, 4, 4), 0),
+    ((20, 40, 48), (1, 1, 1), (10, 10, 10), 0),       # the widest box pitch
+    ((42, 66, 250), (1, 1, 1), (2, 2, 2), 0),         # eight rows per thread in the weight kernel
+])
+def test_paired_form_bit_exact(gpu, port, shape, pr, sr, limit):
+    raw = synth.small_case(shape, seed=sum(shape))
+    sig = _sigmas(shape[0])
+    got, desc = _run(raw, pr, sr, sig, limit)
+    assert "paired" in desc, desc
+    want = port.denoise_f32(raw, FilterParams(search_radius=sr, patch_radius=pr), sig, all_iters=True)
+    assert np.array_equal(got, want), f"{desc}: {np.count_nonzero(got != want)} voxels differ"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pr,sr", [((1, 1, 1), (3, 3, 3)), ((2, 2, 2), (4, 4, 4)), ((3, 3, 3), (2, 2, 2))])
+def test_paired_fused_form_equals_the_other_fused_kernels(gpu, pr, sr):
+    raw = synth.small_case((21, 27, 50), seed=sum(pr) + sum(sr))
+    sig = _sigmas(21)
+    got, desc = _run(raw, pr, sr, sig, precision="f32_fma")
+    assert "paired" in desc and "fused" in desc, desc
+    want, _ = _run(raw, pr, sr, sig, precision="f32_fma", form="tile")
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.gpu
+def test_paired_form_without_room_for_its_workspace(gpu, port):
+    """No workspace (a bound that fits no block, or a failing allocation): the
+    single-pass kernel runs instead, and a later call has its workspace."""
+    L = _lib.load()
+    raw = synth.small_case((20, 24, 40), seed=5)
+    sig = _sigmas(20)
+    want = port.denoise_f32(raw, FilterParams(search_radius=(3, 3, 3), patch_radius=(2, 2, 2)), sig, all_iters=True)
+    got, desc = _run(raw, (2, 2, 2), (3, 3, 3), sig, limit=1000)
+    assert "paired" not in desc, desc
+    assert np.array_equal(got, want)
+    g = IterativeNLM_GPU()
+    g.configure_device(raw.shape, DenoiseParameters(radius_patchspace=(2, 2, 2), radius_searchspace=(3, 3, 3)))
+    for it in range(2):
+        g.set_sigma(sig[it])
+        # iteration 1: the offset table and the z table first, then the workspace
+        L.inlm_debug_fail_allocation(2 if it == 0 else -1)
+        g.Run_GaussianNoise(it + 1, raw if it == 0 else None)
+        L.inlm_debug_fail_allocation(-1)
+        assert np.array_equal(g.get_result(), want[it])
+    assert "paired" in g.describe()
+    g.free_device()
+
+
+@pytest.mark.gpu
+def test_paired_handles_take_turns_on_one_workspace(gpu):
+    L = _lib.load()
+    live = C.c_int64(0)
+    _lib.check(L.inlm_debug_live_allocations(C.byref(live)), "live allocations")
+    before = live.value
+    raw = synth.small_case((16, 24, 40), seed=6)
+    sig = _sigmas(16)
+    shapes = [((1, 1, 1), (4, 4, 4)), ((2, 2, 2), (2, 2, 2))]
+    alone = [_run(raw, pr, sr, sig)[0] for pr, sr in shapes]
+    hs = []
+    for pr, sr in shapes:
+        g = IterativeNLM_GPU()
+        g.configure_device(raw.shape, DenoiseParameters(radius_patchspace=pr, radius_searchspace=sr))
+        hs.append(g)
+    for it in range(2):
+        for g, want in zip(hs, alone):
+            g.set_sigma(sig[it])
+            g.Run_GaussianNoise(it + 1, raw if it == 0 else None)
+            assert np.array_equal(g.get_result(), want[it])
+    for g in hs:
+        g.free_device()
+    _lib.check(L.inlm_debug_live_allocations(C.byref(live)), "live allocations")
+    assert live.value == before
+
+
+@pytest.mark.gpu
+def test_weight_step_equals_the_other_kernels_for_every_argument(gpu):
+    n = C.c_int64(-1)
+    _lib.check(_lib.load().inlm_debug_weight_mismatches(C.byref(n)), "weight_mismatches")
+    assert n.value == 0
+
+
+@pytest.mark.parametrize("pr", [(1, 1, 1), (1, 1, 2), (2, 2, 1), (2, 2, 2), (3, 3, 2), (3, 3, 3)])
+@pytest.mark.parametrize("sr,nslices", [((3, 4, 2), 11), ((5, 5, 5), 7), ((10, 10, 10), 11), ((2, 7, 9), 15)])
+def test_offsets_come_in_mirrored_pairs(lib, pr, sr, nslices):
+    """What the paired form rests on: offset S-1-j is the negative of offset j,
+    z never descends, and a tap's weight depends on |x|, |y|, |z| alone."""
+    cp = DenoiseParameters(radius_patchspace=pr, radius_searchspace=sr, nslices=nslices, z_anisotropy=1.7,
+                           weight_table="distweight").to_c()
+    ns, npatch = C.c_int(0), C.c_int(0)
+    _lib.check(lib.inlm_geometry(C.byref(cp), 40, None, C.byref(ns), None, None, C.byref(npatch), None), "geometry")
+    s, t = np.zeros((ns.value, 3), np.int32), np.zeros((npatch.value, 3), np.int32)
+    w = np.zeros(npatch.value, np.float32)
+    _lib.check(lib.inlm_geometry(C.byref(cp), 40, s.ctypes.data, C.byref(ns), t.ctypes.data, w.ctypes.data,
+                                 C.byref(npatch), None), "geometry")
+    assert np.array_equal(s, -s[::-1]) and (np.diff(s[:, 2]) >= 0).all()
+    by_size = {}
+    for tap, weight in zip(np.abs(t), w):
+        assert by_size.setdefault(tuple(tap), weight) == weight
