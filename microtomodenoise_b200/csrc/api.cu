@@ -265,11 +265,12 @@ int inlm::noise_prepare(inlm_noise* n, const inlm_params* p, int* nwin, bool* fi
             noise_zwindows(n->samples, n->shape, p->zwindow, st, en);
             std::vector<int2> w(nz);
             std::vector<long long> off(nz);
-            long long total = 0;
+            long long total = 0, widest = 0;
             for (int z = 0; z < nz; z++) {
                 w[z] = make_int2(st[z], en[z]);
                 off[z] = total;
                 total += std::max(0, en[z] - st[z] + 1);
+                widest = std::max<long long>(widest, en[z] - st[z] + 1);
             }
             if ((size_t)total > n->assign_cap) {
                 device_free(n->d_assign);
@@ -285,6 +286,7 @@ int inlm::noise_prepare(inlm_noise* n, const inlm_params* p, int* nwin, bool* fi
             CUDA_TRY(cudaStreamSynchronize(n->stream));  // host vectors go out of scope
             n->zwindow_cached = p->zwindow;
             n->mean_window = nz > 0 ? total / nz : 0;
+            n->max_window = widest;
         }
         *nwin = nz;
     } else if (mode == INLM_NOISE_GLOBAL) {
@@ -302,7 +304,7 @@ int inlm::noise_prepare(inlm_noise* n, const inlm_params* p, int* nwin, bool* fi
             CUDA_TRY(cudaMemcpyAsync(n->d_scratch_off, &off, 8, cudaMemcpyHostToDevice, n->stream));
             CUDA_TRY(cudaStreamSynchronize(n->stream));
             n->zwindow_cached = -2;
-            n->mean_window = ns;
+            n->mean_window = n->max_window = ns;
         }
         *nwin = 1;
     }
@@ -313,7 +315,7 @@ int inlm::noise_prepare(inlm_noise* n, const inlm_params* p, int* nwin, bool* fi
 // n->d_sigma (device work only).
 int inlm::noise_em_finish(inlm_noise* n, const inlm_params* p, int nwin) {
     CUDA_TRY(launch_noise_em(n->d_patchstd, n->d_windows, nwin, n->d_scratch_off, n->d_assign,
-                             n->d_mean, n->d_sd, n->stream, n->mean_window));
+                             n->d_mean, n->d_sd, n->stream, n->mean_window, n->max_window));
     CUDA_TRY(launch_noise_finalize(n->d_mean, n->d_sd, n->shape[2],
                                    p->noise_mode == INLM_NOISE_ZADAPTIVE ? 1 : 0, p->stds_from_mean,
                                    n->d_sigma, n->stream));

@@ -123,7 +123,7 @@ static int rgb_noise(RgbJob& J, RgbNoise& N, inlm_params* p, int nx, int ny, int
         return INLM_OK;
     }
     // global two-cluster estimate per channel (z-adaptive is global for one slice)
-    CUDA_TRY(launch_noise_em(J.d_ps, J.d_win, 3, J.d_off, J.d_assign, J.d_mean, J.d_sd, J.st));
+    CUDA_TRY(launch_noise_em(J.d_ps, J.d_win, 3, J.d_off, J.d_assign, J.d_mean, J.d_sd, J.st, 0, ns));
     float mean[3], sd[3];
     CUDA_TRY(cudaMemcpyAsync(mean, J.d_mean, 12, cudaMemcpyDeviceToHost, J.st));
     CUDA_TRY(cudaMemcpyAsync(sd, J.d_sd, 12, cudaMemcpyDeviceToHost, J.st));

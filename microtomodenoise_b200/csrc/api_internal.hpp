@@ -104,6 +104,7 @@ struct inlm_noise {
     float* d_sigma = nullptr;
     int ncalls = 0;
     long long ref_sample_semimanual = 0;
+    long long max_window = 0;   // samples of the largest EM window
     long long mean_window = 0;  // average samples per EM window (picks the EM's CTA size)
 };
 

@@ -10,12 +10,14 @@ cudaError_t launch_noise_patchstd(const float* stack, long long pitch_y, long lo
                                   int patchsize, float* out, cudaStream_t st, int z_base = 0);
 // windows[w] = inclusive sample range; scratch_off[w] = byte offset of the
 // window's assignment array inside scratch.
-// mean_window: average samples per window; from kEmWideWindow on, each window
-// gets a 1024-thread CTA (else 256).
+// max_window: samples of the largest window (0: not known); windows a cluster
+// holds keep their samples in registers and need no scratch. Larger ones:
+// mean_window, the average samples per window; from kEmWideWindow on, each
+// window gets a 1024-thread CTA (else 256).
 constexpr long long kEmWideWindow = 32768;
 cudaError_t launch_noise_em(const float* values, const int2* windows, int n_windows,
                             const long long* scratch_off, signed char* scratch, float* out_mean,
-                            float* out_sd, cudaStream_t st, long long mean_window = 0);
+                            float* out_sd, cudaStream_t st, long long mean_window = 0, long long max_window = 0);
 // Allocation-free EM (static device scratch): limits of the file-scope arrays.
 constexpr long long kNoAllocAssignBytes = 16ll << 20;  // sum of window lengths, samples
 constexpr int kNoAllocMaxWindows = 16384;
