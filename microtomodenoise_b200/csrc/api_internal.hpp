@@ -161,6 +161,7 @@ struct PairRun {
     size_t bytes = 0;       // workspace the plan needs
     void* dist = nullptr;   // borrowed workspace (pair_idle hands it back)
     size_t dist_bytes = 0;
+    bool shared = false;    // bound to a workspace somebody else holds (a batch)
     bool user = false;      // counted among the pool's users
 };
 
@@ -248,6 +249,18 @@ int pair_filter(inlm_denoiser* d);
 void pair_idle(inlm_denoiser* d);
 void pair_release(inlm_denoiser* d);
 bool pair_trim(int device);
+// One workspace for several handles whose passes run one after another (a
+// batch): the bytes a handle's plan needs (0: the form does not run), a loan
+// for the largest, the handles bound to it.
+struct PairLoan {
+    void* p = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+};
+int pair_bytes(inlm_denoiser* d, size_t* bytes);
+int pair_take(int device, size_t bytes, PairLoan* loan);
+void pair_give_back(PairLoan* loan);
+int pair_share(inlm_denoiser* d, void* ws);
 int pad_into(inlm_denoiser* d, const float* src, float* dst);
 int pad_into_half(inlm_denoiser* d, const float* src, void* dst);
 // Noise estimate of a device volume into d_dst (nz floats, device); host_copy

@@ -234,13 +234,36 @@ static int pair_plan(inlm_denoiser* d) {
     return INLM_OK;
 }
 
+// Points the handle's kernels at a workspace of at least r.bytes.
+static int pair_bind(inlm_denoiser* d, void* ws) {
+    PairRun& r = d->pair;
+    PairArgs& a = r.args;
+    if (a.dist == ws) return INLM_OK;  // the tensor maps are this buffer's
+    a.dist = nullptr;
+    const long long pad_dims[3] = {d->nxp, d->nyp, d->nzp}, pad_pitch[2] = {d->pitch_y, d->pitch_z};
+    const int box[3] = {a.pbx, a.pby, a.pbz};
+    int rc = encode_map_f32(&r.maps.prev, d->d_prev_pad, 3, pad_dims, pad_pitch, box);
+    const int obox[4] = {32, 8, 1, 1};
+    const long long dims[4] = {a.ex, a.ey, a.ring, a.H};
+    const long long pitch[3] = {a.ex, (long long)a.ex * a.ey, (long long)a.ex * a.ey * a.ring};
+    if (rc == INLM_OK) rc = encode_map_f32(&r.maps.out, ws, 4, dims, pitch, obox);
+    for (int i = 0; i < 2 && rc == INLM_OK; i++) {
+        const int dbox[4] = {kPairDistBox, pair_weight_rows(i), 1, 1};
+        const int rbox[3] = {a.pbx, pair_weight_rows(i) + 2 * a.syr, 1};
+        rc = encode_map_f32(&r.maps.dist[i], ws, 4, dims, pitch, dbox);
+        if (rc == INLM_OK) rc = encode_map_f32(&r.maps.raw[i], d->d_raw_pad, 3, pad_dims, pad_pitch, rbox);
+    }
+    if (rc) return rc;
+    a.dist = static_cast<float*>(ws);
+    return INLM_OK;
+}
+
 // Borrows a workspace for the handle's next passes; *ok = false where there is
 // no room for one.
 static int pair_borrow(inlm_denoiser* d, bool* ok) {
     PairRun& r = d->pair;
-    PairArgs& a = r.args;
     *ok = true;
-    if (r.dist) return INLM_OK;
+    if (r.dist || r.shared) return INLM_OK;
     if (!r.user) {
         count_user(d->device, 1);
         r.user = true;
@@ -251,24 +274,7 @@ static int pair_borrow(inlm_denoiser* d, bool* ok) {
         *ok = false;
         return INLM_OK;
     }
-    if (a.dist == r.dist) return INLM_OK;  // the tensor maps are this buffer's
-    a.dist = nullptr;
-    const long long pad_dims[3] = {d->nxp, d->nyp, d->nzp}, pad_pitch[2] = {d->pitch_y, d->pitch_z};
-    const int box[3] = {a.pbx, a.pby, a.pbz};
-    int rc = encode_map_f32(&r.maps.prev, d->d_prev_pad, 3, pad_dims, pad_pitch, box);
-    const int obox[4] = {32, 8, 1, 1};
-    const long long dims[4] = {a.ex, a.ey, a.ring, a.H};
-    const long long pitch[3] = {a.ex, (long long)a.ex * a.ey, (long long)a.ex * a.ey * a.ring};
-    if (rc == INLM_OK) rc = encode_map_f32(&r.maps.out, r.dist, 4, dims, pitch, obox);
-    for (int i = 0; i < 2 && rc == INLM_OK; i++) {
-        const int dbox[4] = {kPairDistBox, pair_weight_rows(i), 1, 1};
-        const int rbox[3] = {a.pbx, pair_weight_rows(i) + 2 * a.syr, 1};
-        rc = encode_map_f32(&r.maps.dist[i], r.dist, 4, dims, pitch, dbox);
-        if (rc == INLM_OK) rc = encode_map_f32(&r.maps.raw[i], d->d_raw_pad, 3, pad_dims, pad_pitch, rbox);
-    }
-    if (rc) return rc;
-    a.dist = static_cast<float*>(r.dist);
-    return INLM_OK;
+    return pair_bind(d, r.dist);
 }
 
 // Plans the handle's passes and borrows their workspace; *ready = false when the
@@ -311,6 +317,42 @@ int inlm::pair_filter(inlm_denoiser* d) {
             }
         }
     return INLM_OK;
+}
+
+int inlm::pair_bytes(inlm_denoiser* d, size_t* bytes) {
+    PairRun& r = d->pair;
+    *bytes = 0;
+    if (r.active && !r.planned) {
+        const int rc = pair_plan(d);
+        if (rc) return rc;
+    }
+    if (r.active) *bytes = r.bytes;
+    return INLM_OK;
+}
+
+int inlm::pair_share(inlm_denoiser* d, void* ws) {
+    pair_idle(d);
+    d->pair.shared = true;
+    return pair_bind(d, ws);
+}
+
+int inlm::pair_take(int device, size_t bytes, PairLoan* loan) {
+    count_user(device, 1);
+    if (borrow(device, bytes, &loan->p, &loan->bytes) == cudaSuccess) {
+        loan->device = device;
+        return INLM_OK;
+    }
+    cudaGetLastError();
+    loan->p = nullptr;
+    count_user(device, -1);
+    return INLM_ERR_NOMEM;
+}
+
+void inlm::pair_give_back(PairLoan* loan) {
+    if (!loan->p) return;
+    hand_back(loan->device, loan->p, loan->bytes);
+    count_user(loan->device, -1);
+    loan->p = nullptr;
 }
 
 bool inlm::pair_trim(int device) {
