@@ -156,8 +156,11 @@ static int pair_plan(inlm_denoiser* d) {
     if (r.limit > 0) budget = std::min(budget, r.limit);
     int sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
+    a.dist = nullptr;  // no tensor maps yet
     const int depth = a.nz + a.szc;  // planes whose distances are read
-    const int tz_most = r.tz;
+    const int tz_most = r.tz, rz = g.patch_radius[2];
+    // weight kernel's time over distance kernel's (measured: 1.2, 0.6, 0.25)
+    const double weights_share = g.patch_radius[0] == 1 ? 1.2 : g.patch_radius[0] == 2 ? 0.6 : 0.25;
     double best = 0;
     for (int nby = 1; nby <= 32; nby++)
         for (int nbx = 1; nbx <= 32; nbx++) {
@@ -167,35 +170,38 @@ static int pair_plan(inlm_denoiser* d) {
             const int tiles_y = (2 * a.syr + std::min(by, a.ny) + 7) / 8;
             const size_t plane = (size_t)tiles_x * 32 * tiles_y * 8 * a.H * 4;
             const int ring_max = (int)std::min<size_t>(budget / plane, 1 << 20);
-            int chunk = depth, ring = depth, tz = tz_most;
-            if (ring > ring_max) {
-                // as few chunks of whole tiles as fit, or tiles as deep as fit
-                tz = std::min(tz, ring_max - a.szc);
-                if (tz < 4) continue;
-                chunk = (ring_max - a.szc) / tz * tz;
-                const int n = (depth + chunk - 1) / chunk;
-                chunk = round_up((depth + n - 1) / n, tz);
-                ring = chunk + a.szc;
-            }
-            const int tiles_z = (chunk + tz - 1) / tz, n_chunks = (depth + chunk - 1) / chunk;
-            // tiles of all launches, and a third of a wave of tiles lost at
-            // the end of each
-            const double tiles = (double)tiles_x * tiles_y * tiles_z;
-            // (a tile of tz planes walks tz + 2 RZ)
-            const double cost = (tiles / sms + 0.3) * (tz + 2 * g.patch_radius[2]) * n_chunks * nbx * nby;
-            if (best == 0 || cost < best) {
-                best = cost;
-                r.bx = bx;
-                r.by = by;
-                r.chunk = chunk;
-                a.tz = tz;
-                a.pbz = tz + 2 * g.patch_radius[2] + a.szc;
-                a.tiles_x = tiles_x;
-                a.tiles_y = tiles_y;
-                a.ex = tiles_x * 32;
-                a.ey = tiles_y * 8;
-                a.ring = ring;
-            }
+            // the whole volume where it fits, else chunks of k layers of tiles
+            // of any depth down to half the deepest
+            const bool whole = depth <= ring_max;
+            for (int k = 1; k <= (whole ? 1 : 64); k++)
+                for (int tz = tz_most; tz >= (whole ? tz_most : std::max(4, tz_most / 2)); tz--) {
+                    const int chunk = whole ? depth : std::min(depth, k * tz), ring = whole ? depth : chunk + a.szc;
+                    if (ring > ring_max) continue;
+                    const int n_chunks = (depth + chunk - 1) / chunk;
+                    // distances: tiles of all launches (a tile of tz planes
+                    // walks tz + 2 RZ), and a third of a wave of tiles lost per
+                    // launch; weights: whole waves of CTAs (four per SM), at the
+                    // share of the time that they take
+                    const double layers = (double)((chunk + tz - 1) / tz) * n_chunks;
+                    const double walk = (double)tiles_x * tiles_y * layers / sms * (tz + 2 * rz) +
+                                        0.3 * n_chunks * (tz_most + 2 * rz);
+                    const double ctas = (double)((std::min(bx, a.nx) + 31) / 32) * ((std::min(by, a.ny) + 31) / 32) *
+                                        std::min(chunk, a.nz) / (4.0 * sms);
+                    const double cost = walk * (1.0 + weights_share * std::ceil(ctas) / ctas) * nbx * nby;
+                    if (best == 0 || cost < best) {
+                        best = cost;
+                        r.bx = bx;
+                        r.by = by;
+                        r.chunk = chunk;
+                        a.tz = tz;
+                        a.pbz = tz + 2 * rz + a.szc;
+                        a.tiles_x = tiles_x;
+                        a.tiles_y = tiles_y;
+                        a.ex = tiles_x * 32;
+                        a.ey = tiles_y * 8;
+                        a.ring = ring;
+                    }
+                }
         }
     if (best == 0) {
         r.active = false;
