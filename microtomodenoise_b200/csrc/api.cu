@@ -992,7 +992,7 @@ extern "C" int inlm_denoiser_create(const int shape[3], const inlm_params* p, in
     if (e != cudaSuccess) return bail(fail(INLM_ERR_CUDA, "stream: %s", cudaGetErrorString(e)));
     d->own_stream = true;
     if (dalloc(&d->d_next, nvox) != cudaSuccess || dalloc(&d->d_sigma, shape[2]) != cudaSuccess ||
-        dalloc(&d->d_sigma0, shape[2]) != cudaSuccess || dalloc(&d->d_mult, shape[2]) != cudaSuccess ||
+        dalloc(&d->d_sigma0, 2 * (size_t)shape[2]) != cudaSuccess || dalloc(&d->d_mult, shape[2]) != cudaSuccess ||
         dalloc(&d->d_err, 1) != cudaSuccess || cudaMemset(d->d_err, 0, 4) != cudaSuccess)
         return bail(fail(INLM_ERR_NOMEM, "device allocation failed"));
     if (f16) {
@@ -1356,8 +1356,7 @@ extern "C" int inlm_denoise(inlm_denoiser* d, const float* raw, float* out, int 
         raw_dev = d->d_next;
     }
     // sigma0 on the raw data (main.cpp:327-351)
-    std::vector<float> s0h, s1h;
-    int rc = estimate_into(d, raw_dev, d->d_sigma0, sigma0_out ? &s0h : nullptr);
+    int rc = estimate_into(d, raw_dev, d->d_sigma0, nullptr);
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(d->d_sigma, d->d_sigma0, nz * 4, cudaMemcpyDeviceToDevice, d->stream));
     rc = upload_sigma_device(d);
@@ -1367,8 +1366,12 @@ extern "C" int inlm_denoise(inlm_denoiser* d, const float* raw, float* out, int 
     const int maxit = d->p.maxiterations;
     if (maxit > 1) {
         // sigma1 on the first result, blended with sigma0 (main.cpp:422-448)
-        rc = estimate_into(d, d->d_next, d->d_sigma, sigma1_out ? &s1h : nullptr);
+        rc = estimate_into(d, d->d_next, d->d_sigma, nullptr);
         if (rc) return rc;
+        // the pre-blend estimate is what the reference reports (main.cpp:438);
+        // it is kept behind sigma0, and the host reads both when the job is
+        // done: a copy to pageable memory here would hold up the launches
+        CUDA_TRY(cudaMemcpyAsync(d->d_sigma0 + nz, d->d_sigma, nz * 4, cudaMemcpyDeviceToDevice, d->stream));
         CUDA_TRY(launch_sigma_blend(d->d_sigma0, d->d_sigma, d->p.alpha, nz, d->stream));
         d->launches++;
         rc = upload_sigma_device(d);
@@ -1392,13 +1395,14 @@ extern "C" int inlm_denoise(inlm_denoiser* d, const float* raw, float* out, int 
     } else {
         CUDA_TRY(cudaMemcpyAsync(out, d->d_next, nvox * 4, cudaMemcpyDeviceToHost, d->stream));
     }
-    CUDA_TRY(cudaStreamSynchronize(d->stream));
-    if (sigma0_out) std::memcpy(sigma0_out, s0h.data(), nz * 4);
-    if (sigma1_out && maxit > 1) {
-        // the pre-blend estimate is what the reference reports (main.cpp:438)
-        std::memcpy(sigma1_out, s1h.data(), nz * 4);
-    }
-    return check_device_error(d);
+    std::vector<float> sigmas(2 * (size_t)nz);
+    if (sigma0_out || (sigma1_out && maxit > 1))
+        CUDA_TRY(cudaMemcpyAsync(sigmas.data(), d->d_sigma0, (maxit > 1 ? 2 : 1) * nz * 4, cudaMemcpyDeviceToHost,
+                                 d->stream));
+    rc = check_device_error(d);  // and the stream has drained
+    if (sigma0_out) std::copy(sigmas.begin(), sigmas.begin() + nz, sigma0_out);
+    if (sigma1_out && maxit > 1) std::copy(sigmas.begin() + nz, sigmas.end(), sigma1_out);
+    return rc;
 }
 
 extern "C" int inlm_filter_kernel_ms(inlm_denoiser* d, double* avg_ms, int* n_launches) {

@@ -178,7 +178,7 @@ struct inlm_denoiser {
     float* d_prev_pad = nullptr;
     float* d_next = nullptr;
     float* d_sigma = nullptr;
-    float* d_sigma0 = nullptr;
+    float* d_sigma0 = nullptr;  // nz values, and behind them the pre-blend sigma1 of the job
     float* d_mult = nullptr;
     int* d_err = nullptr;
     int2* d_search_delta = nullptr;

@@ -89,6 +89,15 @@ int offset_splits(int tiles, int sms, int most) {
     return best;
 }
 
+// Plane steps of the longest-working warp of a launch (the kernel's split of
+// whole offsets and of the rest among its warps).
+double warp_steps(int tiles, int splits, int sms, int warps, int H, int tz, int rz) {
+    const int lanes = warps * splits, rest = H % lanes;
+    const int parts = rest ? std::max(1, std::min(lanes / rest, tz / (2 * rz + 2))) : 1;
+    const double rounds = (double)(H / lanes) * (tz + 2 * rz) + (rest ? (double)tz / parts + 2 * rz : 0.0);
+    return rounds * ((tiles * (long long)splits + sms - 1) / sms);
+}
+
 }  // namespace
 
 // Whether the paired form covers the handle's configuration: an instantiated
@@ -207,6 +216,23 @@ static int pair_plan(inlm_denoiser* d) {
         r.active = false;
         return INLM_OK;
     }
+    r.sms = sms;
+    r.warps = pair_kernel_warps(g.patch_radius[0]);
+    // a volume that leaves SMs idle even with its offsets shared out: shallower
+    // tiles, whose walks are shorter
+    const int most = (a.H + r.warps - 1) / r.warps;
+    if (r.chunk == depth && a.tiles_x * a.tiles_y * ((depth + a.tz - 1) / a.tz) * most < sms) {
+        double least = 0;
+        for (int tz = tz_most; tz >= 4; tz--) {
+            const int tiles = a.tiles_x * a.tiles_y * ((depth + tz - 1) / tz);
+            const double steps = warp_steps(tiles, offset_splits(tiles, sms, most), sms, r.warps, a.H, tz, rz);
+            if (least == 0 || steps < least) {
+                least = steps;
+                a.tz = tz;
+                a.pbz = tz + 2 * rz + a.szc;
+            }
+        }
+    }
     const int S = a.S;
     std::vector<PairOffset> t(S);
     for (int s = 0; s < S; s++) {
@@ -234,8 +260,6 @@ static int pair_plan(inlm_denoiser* d) {
     a.out = d->d_next;
     a.mult = d->d_mult;
     a.err = d->d_err;
-    r.sms = sms;
-    r.warps = pair_kernel_warps(g.patch_radius[0]);
     r.planned = true;
     return INLM_OK;
 }

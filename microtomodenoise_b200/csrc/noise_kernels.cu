@@ -745,8 +745,9 @@ cudaError_t launch_noise_em(const float* values, const int2* windows, int n_wind
     if (max_window > 0 && max_window <= (long long)kEmMaxCluster * kEmClusterThreads * kEmMaxValues) {
         int ctas = 1;
         while ((long long)ctas * kEmClusterThreads * kEmMaxValues < max_window) ctas *= 2;
+        // (a barrier of the cluster costs as much as a dozen samples per thread)
         while (ctas < kEmMaxCluster && (long long)n_windows * ctas * 2 <= 148 &&
-               (long long)ctas * kEmClusterThreads * 4 < max_window)
+               (long long)ctas * kEmClusterThreads * 12 < max_window)
             ctas *= 2;
         const long long per = (max_window + (long long)ctas * kEmClusterThreads - 1) / ((long long)ctas * kEmClusterThreads);
         if (per <= 4) return launch_em_cluster<4>(values, windows, n_windows, ctas, out_mean, out_sd, st);
