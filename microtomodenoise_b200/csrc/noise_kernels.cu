@@ -265,7 +265,7 @@ __device__ __forceinline__ void em_window(const float* __restrict__ values, int 
 // in every pass, a decision takes a dozen FP32 operations, and a reduction is
 // one warp-shuffle tree, one barrier in the CTA and one in the cluster. A global
 // estimate of 100000 samples takes 0.21 ms (one 1024-thread CTA: 2.49 ms), 256
-// windows of up to 39000 samples 0.79 ms (1.67 ms), 4000 samples 0.060 ms (0.18 ms).
+// windows of up to 39000 samples 0.73 ms (1.67 ms), 4000 samples 0.060 ms (0.18 ms).
 //
 // Decision: p2 > p1 with p = float(1/sqrt(2 pi var) * expf(-q)) as cluster_prob
 // rounds it. In logarithms that is t = q1 - q2 + ln(var1/var2)/2 > 0, and every
@@ -274,6 +274,7 @@ __device__ __forceinline__ void em_window(const float* __restrict__ values, int 
 // number, its sign decides; any other sample (near a tie, an underflow, a NaN)
 // takes cluster_prob itself.
 constexpr int kEmClusterThreads = 512;
+constexpr int kEmManyThreads = 256, kEmManyValues = 40;  // the shape for many windows
 constexpr int kEmMaxCluster = 8;
 constexpr int kEmMaxValues = 28;  // per thread (64 registers at two CTAs per SM)
 
@@ -286,13 +287,13 @@ struct __align__(16) EmPartial {
 // an order that depends on nothing but the launch; all threads of all its CTAs
 // call it and get the result. The two sums share one shuffle tree: lanes 0-15
 // carry s1, lanes 16-31 s2.
-template <bool COUNTS>
+template <int NT, bool COUNTS>
 __device__ __forceinline__ void cluster_sum(EmPartial& r, EmPartial* warp_part, EmPartial (*slots)[kEmMaxCluster],
                                             int& parity, int ctas, unsigned rank) {
     namespace cg = cooperative_groups;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int NW = kEmClusterThreads / 32;
-    static_assert(NW == 16, "one partial per lane of a half warp");
+    constexpr int NW = NT / 32;
+    static_assert(NW <= 16, "one partial per lane of a half warp");
     const bool low = lane < 16;
     double x = (low ? r.s1 : r.s2) + __shfl_xor_sync(0xffffffffu, low ? r.s2 : r.s1, 16);
 #pragma unroll
@@ -307,13 +308,13 @@ __device__ __forceinline__ void cluster_sum(EmPartial& r, EmPartial* warp_part, 
     if (lane == 0) part[warp].s1 = x;
     if (lane == 16) part[warp].s2 = x;
     __syncthreads();
-    x = low ? part[lane].s1 : part[lane - 16].s2;
+    x = (lane & 15) >= NW ? 0.0 : low ? part[lane].s1 : part[lane - 16].s2;
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     r.s1 = __shfl_sync(0xffffffffu, x, 0);
     r.s2 = __shfl_sync(0xffffffffu, x, 16);
     if (COUNTS) {
-        const int4 c = low ? *reinterpret_cast<const int4*>(&part[lane].n1) : make_int4(0, 0, 0, 0);
+        const int4 c = lane < NW ? *reinterpret_cast<const int4*>(&part[lane].n1) : make_int4(0, 0, 0, 0);
         r.n1 = __reduce_add_sync(0xffffffffu, c.x);
         r.n2 = __reduce_add_sync(0xffffffffu, c.y);
         r.flag = __any_sync(0xffffffffu, c.z);
@@ -344,11 +345,33 @@ __device__ __forceinline__ float2 quotients(double s1, double s2, int n1, int n2
     return make_float2(__shfl_sync(0xffffffffu, f, 0), __shfl_sync(0xffffffffu, f, 16));
 }
 
-template <int VPT>
-__global__ void __launch_bounds__(kEmClusterThreads, 2)
+// One bit per sample of a thread.
+template <int N>
+struct Bits {
+    unsigned w[(N + 31) / 32];
+    __device__ __forceinline__ bool operator[](int k) const { return w[k / 32] >> (k % 32) & 1u; }
+    __device__ __forceinline__ void set(int k) { w[k / 32] |= 1u << (k % 32); }
+    __device__ __forceinline__ void put(int k, bool b) { w[k / 32] = (w[k / 32] & ~(1u << (k % 32))) | (unsigned)b << (k % 32); }
+    template <class F>
+    __device__ __forceinline__ static Bits map(F f) {
+        Bits r;
+#pragma unroll
+        for (int i = 0; i < (N + 31) / 32; i++) r.w[i] = f(i);
+        return r;
+    }
+    __device__ __forceinline__ int count() const {
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < (N + 31) / 32; i++) n += __popc(w[i]);
+        return n;
+    }
+};
+
+template <int NT, int VPT>
+__global__ void __launch_bounds__(NT, NT == kEmManyThreads ? 3 : 2)
     noise_em_cluster_kernel(const float* __restrict__ values, const int2* __restrict__ windows, int ctas,
                             float* __restrict__ out_mean, float* __restrict__ out_sd) {
-    constexpr int NT = kEmClusterThreads;
+    using B = Bits<VPT>;
     __shared__ EmPartial warp_part[2 * NT / 32];
     __shared__ EmPartial slots[2][kEmMaxCluster];
     __shared__ float range_part[2][2 * NT / 32];
@@ -360,7 +383,7 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int stride = NT * ctas;
     float v[VPT];
-    unsigned in = 0;    // samples of the window that are not zero
+    B in = B::map([](int) { return 0u; });  // samples of the window that are not zero
     bool odd = false;   // one of them is not a number
     float mn = 1e20f, mx = -1e20f;
 #pragma unroll
@@ -371,7 +394,7 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
             v[k] = values[i];
             mn = fminf(mn, v[k]);
             mx = fmaxf(mx, v[k]);
-            if (v[k] != 0.0f) in |= 1u << k;
+            if (v[k] != 0.0f) in.set(k);
             odd |= v[k] != v[k];
         }
     }
@@ -409,31 +432,31 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
 
     // initial assignment, zero values excluded (noiselevel.cpp:398-423)
     int parity = 0;
-    unsigned two = 0;  // samples of the second cluster
+    B two = B::map([](int) { return 0u; });  // samples of the second cluster
     EmPartial r;
     // the thread's cluster sums and counts under the assignment `two`
     auto sums = [&]() {
         double s1 = 0.0, s2 = 0.0;
-        const unsigned first = in & ~two;
+        const B first = B::map([&](int i) { return in.w[i] & ~two.w[i]; });
 #pragma unroll
         for (int k = 0; k < VPT; k++) {
             const double d = (double)v[k];
-            if (two >> k & 1u) s2 += d;
-            if (first >> k & 1u) s1 += d;
+            if (two[k]) s2 += d;
+            if (first[k]) s1 += d;
         }
         r.s1 = s1;
         r.s2 = s2;
-        r.n1 = __popc(first);
-        r.n2 = __popc(two);
+        r.n1 = first.count();
+        r.n2 = two.count();
     };
 #pragma unroll
     for (int k = 0; k < VPT; k++)
-        if (!(fabsf(__fsub_rn(v[k], mean1)) < fabsf(__fsub_rn(v[k], mean2)))) two |= 1u << k;
-    two &= in;
+        if (!(fabsf(__fsub_rn(v[k], mean1)) < fabsf(__fsub_rn(v[k], mean2)))) two.set(k);
+    two = B::map([&](int i) { return two.w[i] & in.w[i]; });
     r.flag = 0;
     sums();
     double own1 = r.s1, own2 = r.s2;
-    cluster_sum<true>(r, warp_part, slots, parity, ctas, rank);
+    cluster_sum<NT, true>(r, warp_part, slots, parity, ctas, rank);
     float2 mean = quotients(r.s1, r.s2, r.n1, r.n2);
     if (r.n1 > 0) mean1 = mean.x;
     if (r.n2 > 0) mean2 = mean.y;
@@ -449,19 +472,19 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
     float var1, var2;
     auto variances = [&]() {
         double s1 = 0.0, s2 = 0.0;
-        const unsigned first = in & ~two;
+        const B first = B::map([&](int i) { return in.w[i] & ~two.w[i]; });
 #pragma unroll
         for (int k = 0; k < VPT; k++) {
-            const bool b = two >> k & 1u;
+            const bool b = two[k];
             const float d = __fsub_rn(v[k], b ? mean2 : mean1);
             const double q = (double)__fmul_rn(d, d);
             if (b) s2 += q;
-            if (first >> k & 1u) s1 += q;
+            if (first[k]) s1 += q;
         }
         EmPartial q;
         q.s1 = s1;
         q.s2 = s2;
-        cluster_sum<false>(q, warp_part, slots, parity, ctas, rank);
+        cluster_sum<NT, false>(q, warp_part, slots, parity, ctas, rank);
         const float2 var = quotients(q.s1, q.s2, max(n1, 1), max(n2, 1));
         var1 = var.x;
         var2 = var.y;
@@ -481,7 +504,7 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
         const bool safe = fmaxf(fmaxf(fminf(q(mn, mean1, r1), q(mn, mean2, r2)),
                                       fminf(q(mx, mean1, r1), q(mx, mean2, r2))),
                                 fminf(q(mean2, mean1, r1), q(mean1, mean2, r2))) < 80.f;
-        unsigned one = 0;
+        B one = B::map([](int) { return 0u; });
         float nearest = 1e30f;
 #pragma unroll
         for (int k = VPT - 1; k >= 0; k--) {
@@ -489,21 +512,25 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
             const float q1 = d1 * d1 * r1, q2 = d2 * d2 * r2;
             const float t = q1 - q2 + shift;
             nearest = fminf(nearest, fmaf(-2e-6f, q1 + q2, fabsf(t)));
-            one = __funnelshift_l(__float_as_uint(t), one, 1);  // bit k: t < 0
+            one.w[k / 32] = __funnelshift_l(__float_as_uint(t), one.w[k / 32], 1);  // bit k: t < 0
         }
-        unsigned next = ~one;
+        B next = B::map([&](int i) { return ~one.w[i]; });
         if (!(nearest > slack) || !safe || odd) {
             for (int k = 0; k < VPT; k++) {
                 const float x = values[min(fs + (int)rank * NT + tid + k * stride, ls)];
                 const float q1 = q(x, mean1, r1), q2 = q(x, mean2, r2);
                 if (safe && fmaf(-2e-6f, q1 + q2, fabsf(q1 - q2 + shift)) > 2.f * slack) continue;
                 const bool b = cluster_prob(x, mean2, var2) > cluster_prob(x, mean1, var1);
-                next = (next & ~(1u << k)) | (unsigned)b << k;
+                next.put(k, b);
             }
         }
-        next &= in;
-        r.flag = next != two;
-        if (next != two) {
+        r.flag = 0;
+#pragma unroll
+        for (int i = 0; i < (VPT + 31) / 32; i++) {
+            next.w[i] &= in.w[i];
+            r.flag |= next.w[i] != two.w[i];
+        }
+        if (r.flag) {
             two = next;
             sums();
             own1 = r.s1;
@@ -511,9 +538,9 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
         }
         r.s1 = own1;
         r.s2 = own2;
-        r.n1 = __popc(in & ~two);
-        r.n2 = __popc(two);
-        cluster_sum<true>(r, warp_part, slots, parity, ctas, rank);
+        r.n1 = in.count() - two.count();  // two lies in in
+        r.n2 = two.count();
+        cluster_sum<NT, true>(r, warp_part, slots, parity, ctas, rank);
         change = r.flag;
         n1 = r.n1;
         n2 = r.n2;
@@ -533,12 +560,12 @@ __global__ void __launch_bounds__(kEmClusterThreads, 2)
     }
 }
 
-template <int VPT>
+template <int NT, int VPT>
 static cudaError_t launch_em_cluster(const float* values, const int2* windows, int n_windows, int ctas,
                                      float* out_mean, float* out_sd, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(n_windows * ctas);
-    cfg.blockDim = dim3(kEmClusterThreads);
+    cfg.blockDim = dim3(NT);
     cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -546,7 +573,7 @@ static cudaError_t launch_em_cluster(const float* values, const int2* windows, i
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, noise_em_cluster_kernel<VPT>, values, windows, ctas, out_mean, out_sd);
+    return cudaLaunchKernelEx(&cfg, noise_em_cluster_kernel<NT, VPT>, values, windows, ctas, out_mean, out_sd);
 }
 
 template <int NT>
@@ -744,16 +771,24 @@ cudaError_t launch_noise_em(const float* values, const int2* windows, int n_wind
     // idle SMs: a pass is then shorter
     if (max_window > 0 && max_window <= (long long)kEmMaxCluster * kEmClusterThreads * kEmMaxValues) {
         int ctas = 1;
+        // many windows: half the threads with more samples each, so that the
+        // reductions take fewer of the issue slots (256 windows of up to 39000
+        // samples: 727 us against 794 us)
+        while ((long long)ctas * kEmManyThreads * kEmManyValues < max_window) ctas *= 2;
+        if (ctas <= kEmMaxCluster && (long long)n_windows * ctas >= 4 * 148 &&
+            max_window > (long long)ctas * kEmManyThreads * kEmManyValues / 2)
+            return launch_em_cluster<kEmManyThreads, kEmManyValues>(values, windows, n_windows, ctas, out_mean, out_sd, st);
+        ctas = 1;
         while ((long long)ctas * kEmClusterThreads * kEmMaxValues < max_window) ctas *= 2;
         // (a barrier of the cluster costs as much as a dozen samples per thread)
         while (ctas < kEmMaxCluster && (long long)n_windows * ctas * 2 <= 148 &&
                (long long)ctas * kEmClusterThreads * 12 < max_window)
             ctas *= 2;
         const long long per = (max_window + (long long)ctas * kEmClusterThreads - 1) / ((long long)ctas * kEmClusterThreads);
-        if (per <= 4) return launch_em_cluster<4>(values, windows, n_windows, ctas, out_mean, out_sd, st);
-        if (per <= 12) return launch_em_cluster<12>(values, windows, n_windows, ctas, out_mean, out_sd, st);
-        if (per <= 20) return launch_em_cluster<20>(values, windows, n_windows, ctas, out_mean, out_sd, st);
-        return launch_em_cluster<kEmMaxValues>(values, windows, n_windows, ctas, out_mean, out_sd, st);
+        if (per <= 4) return launch_em_cluster<kEmClusterThreads, 4>(values, windows, n_windows, ctas, out_mean, out_sd, st);
+        if (per <= 12) return launch_em_cluster<kEmClusterThreads, 12>(values, windows, n_windows, ctas, out_mean, out_sd, st);
+        if (per <= 20) return launch_em_cluster<kEmClusterThreads, 20>(values, windows, n_windows, ctas, out_mean, out_sd, st);
+        return launch_em_cluster<kEmClusterThreads, kEmMaxValues>(values, windows, n_windows, ctas, out_mean, out_sd, st);
     }
     // long windows (few of them, e.g. a global estimate or a short stack) get
     // 1024 threads each so one CTA per window still keeps an SM busy

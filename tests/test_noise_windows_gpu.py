@@ -1,5 +1,5 @@
 """EM window sizes at which the device estimator changes its form: samples per
-thread (4, 12, 20, 28), CTAs per cluster (1, 2, 4, 8) and the scratch form for
+thread (4, 12, 20, 28, 40), CTAs per cluster (1, 2, 4, 8) and the scratch form for
 windows no cluster holds, with zero samples and near-ties among them."""
 import numpy as np
 import pytest
@@ -22,7 +22,18 @@ REL_TOL = 1e-6
 ])
 @pytest.mark.parametrize("flat", [False, True])
 def test_sigma_at_every_window_form(gpu, port, n, mode, zwindow, flat):
-    vol = synth.small_case((20, 40, 48), seed=n % 97)
+    _check(port, (20, 40, 48), n, mode, zwindow, flat)
+
+
+@pytest.mark.parametrize("n,zwindow", [(40000, 20), (40000, 140), (60000, 140), (100000, 190)])
+def test_sigma_with_many_windows(gpu, port, n, zwindow):
+    """Hundreds of slices: the shape with more samples per thread, from half
+    full on."""
+    _check(port, (600, 17, 18), n, "z-adaptive", zwindow, False)
+
+
+def _check(port, shape, n, mode, zwindow, flat):
+    vol = synth.small_case(shape, seed=n % 97)
     if flat:
         vol[:, :24] = 0.5  # patches of std 0 are excluded, whole windows may be empty
         vol[7:11] = 0.25
