@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "filter_fast.cuh"
+#include "pair_math.cuh"
 #include "tile_common.cuh"
 
 namespace inlm {
@@ -220,6 +221,13 @@ __global__ void __launch_bounds__(TX * TZ * 8 / FastThreads<TX>::VPT, TX == 32 ?
     using F = FastGeom<RX, RY, RZ, TZ, TX, D_HALF>;
     constexpr int VPT = FastThreads<TX>::VPT;
     constexpr int NT = TX * TZ * 8 / VPT;  // threads
+    // Squared differences and weights in f32x2 pairs, with the same roundings.
+    // Issue slots bound the half2 form, and pairs spare 8 of about 55 per voxel
+    // and offset: 256 x 256 x 128, patch radius 2, search radius 5 13.0 -> 12.2
+    // ms. With FP32 planes (17.5 -> 18.1 ms) and at patch radius 3 (203 x 187 x
+    // 61, search radius 7: 26.5 -> 27.3 ms) the FP32 lanes and the larger
+    // bodies' registers bound it, and scalars stay.
+    constexpr bool PACKED = D_HALF && !MASS && RX <= 2;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
     __half* prevb = reinterpret_cast<__half*>(smem + 128);
@@ -307,17 +315,33 @@ __global__ void __launch_bounds__(TX * TZ * 8 / FastThreads<TX>::VPT, TX == 32 ?
         og1[k] = __half2float(prevb[qpi[k] + 1]);
     }
 
+    // Every pair of a thread starts on an even column of the D plane, and the
+    // box pitches are even, so the parity of the pair's box index is that of
+    // px - RX + dlx: where it is even the pair is one 32-bit load.
     auto phase_a = [&](unsigned char* Dw, int dlx) {
-#pragma unroll
-        for (int k = 0; k < NQ; k++) {
-            float t0 = __half2float(prevb[qpi[k] + dlx]) - og0[k];
-            float t1 = __half2float(prevb[qpi[k] + dlx + 1]) - og1[k];
-            float d0 = (t0 * scale) * t0, d1 = (t1 * scale) * t1;
-            if constexpr (D_HALF) {
-                reinterpret_cast<__half2*>(Dw)[qdi[k] / 2] = __floats2half2_rn(d0, d1);
+        auto put = [&](int k, float2 v) {
+            float2 d;
+            if constexpr (PACKED) {
+                const f32x2 t = sub2(pack2(v.x, v.y), pack2(og0[k], og1[k]));
+                d = unpack2(mul2_to_mul(mul2_to_mul(t, splat2(scale)), t));
             } else {
-                reinterpret_cast<float2*>(Dw)[qdi[k] / 2] = make_float2(d0, d1);
+                const float t0 = v.x - og0[k], t1 = v.y - og1[k];
+                d = make_float2((t0 * scale) * t0, (t1 * scale) * t1);
             }
+            if constexpr (D_HALF) {
+                reinterpret_cast<__half2*>(Dw)[qdi[k] / 2] = __floats2half2_rn(d.x, d.y);
+            } else {
+                reinterpret_cast<float2*>(Dw)[qdi[k] / 2] = d;
+            }
+        };
+        if (PACKED && ((a.px - RX + dlx) & 1) == 0) {
+#pragma unroll
+            for (int k = 0; k < NQ; k++)
+                put(k, __half22float2(*reinterpret_cast<const __half2*>(prevb + qpi[k] + dlx)));
+        } else {
+#pragma unroll
+            for (int k = 0; k < NQ; k++)
+                put(k, make_float2(__half2float(prevb[qpi[k] + dlx]), __half2float(prevb[qpi[k] + dlx + 1])));
         }
     };
 
@@ -409,25 +433,45 @@ __global__ void __launch_bounds__(TX * TZ * 8 / FastThreads<TX>::VPT, TX == 32 ?
                     tile_distances<RX, RY, RZ, TZ, TX, D_HALF, VPT, 0>(Dr, rowoff, dist, a);
                 }
                 float part = 0.0f;
+                if constexpr (PACKED) {
+                    const f32x2 rel2 = splat2(rel);
 #pragma unroll
-                for (int r = 0; r < VPT; r++) {
-                    const float x = dist[r] * rel;
-                    // Pade[3/3] of exp in Horner form, FMA
-                    const float num = fmaf(fmaf(x + 12.f, x, 60.f), x, 120.f);
-                    const float den = fmaf(fmaf(12.f - x, x, -60.f), x, 120.f);
-                    const float q = __fdividef(num, den);  // formed, then selected
-                    const float w = (x > -3.56648f) ? q : 0.0f;
-                    if constexpr (MASS) {
-                        part = fmaf(w, inv[r], part);
-                    } else {
-                        float rs;
+                    for (int r = 0; r < VPT; r += 2) {
+                        float2 rs;
                         if constexpr (RAW_G)
-                            rs = rcur[r];
+                            rs = make_float2(rcur[r], rcur[r + 1]);
                         else
-                            rs = __half2float(rsrc_v[rbase + dly + r]);
-                        acc[r] = fmaf(w, rs, acc[r]);
-                        wsum[r] += w;
-                        wmax[r] = fmaxf(wmax[r], w);
+                            rs = make_float2(__half2float(rsrc_v[rbase + dly + r]),
+                                             __half2float(rsrc_v[rbase + dly + r + 1]));
+                        f32x2 ac = pack2(acc[r], acc[r + 1]), ws = pack2(wsum[r], wsum[r + 1]);
+                        fused_weight_pair(pack2(dist[r], dist[r + 1]), rel2, rs, ac, ws, wmax[r], wmax[r + 1]);
+                        const float2 au = unpack2(ac), wu = unpack2(ws);
+                        acc[r] = au.x;
+                        acc[r + 1] = au.y;
+                        wsum[r] = wu.x;
+                        wsum[r + 1] = wu.y;
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < VPT; r++) {
+                        const float x = dist[r] * rel;
+                        // Pade[3/3] of exp in Horner form, FMA
+                        const float num = fmaf(fmaf(x + 12.f, x, 60.f), x, 120.f);
+                        const float den = fmaf(fmaf(12.f - x, x, -60.f), x, 120.f);
+                        const float q = __fdividef(num, den);  // formed, then selected
+                        const float w = (x > -3.56648f) ? q : 0.0f;
+                        if constexpr (MASS) {
+                            part = fmaf(w, inv[r], part);
+                        } else {
+                            float rs;
+                            if constexpr (RAW_G)
+                                rs = rcur[r];
+                            else
+                                rs = __half2float(rsrc_v[rbase + dly + r]);
+                            acc[r] = fmaf(w, rs, acc[r]);
+                            wsum[r] += w;
+                            wmax[r] = fmaxf(wmax[r], w);
+                        }
                     }
                 }
                 if constexpr (MASS) {
