@@ -752,10 +752,11 @@ int inlm::tile_config_try(inlm_denoiser* d, int tz, bool raw_smem, bool* ok, boo
 
 // The single-pass kernel (before any autotuning): the first candidate that
 // fits. It runs where the paired form (api_pair.cu) does not: no workspace, a
-// form selected by name, the batch. Everywhere else the paired form is faster,
-// measured over patch shapes, search radii 2 to 10 and 36 volumes of 27 thousand to 18
-// million voxels: 1.02 to 1.4 times at patch radius 1 (fused: 1.0 to 1.2), 1.7
-// to 2.7 times at radius 2 and 3, more where few tiles leave SMs idle.
+// form selected by name, small volumes of a batch, the fused form at patch radius
+// 1 on volumes that fill the SMs. Everywhere else the paired form is faster,
+// measured over patch shapes, search radii 2 to 10 and 36 volumes of 27 thousand
+// to 18 million voxels: 1.02 to 1.4 times at patch radius 1, 1.7 to 2.7 times at
+// radius 2 and 3, more where few tiles leave SMs idle.
 // form: 0 every candidate, 1 the tiled kernels only, 2 the column form only,
 // 3 the warp-specialised kernel only. In form 0 the warp-specialised kernel
 // leads when patch sums dominate the work (at least 100 patch taps, or at

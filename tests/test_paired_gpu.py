@@ -145,3 +145,23 @@ def test_offsets_come_in_mirrored_pairs(lib, pr, sr, nslices):
     by_size = {}
     for tap, weight in zip(np.abs(t), w):
         assert by_size.setdefault(tuple(tap), weight) == weight
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,paired", [((17, 40, 64), True), ((65, 72, 127), False)])
+def test_fused_patch_radius_1_runs_the_column_form_on_volumes_that_fill_the_gpu(gpu, shape, paired):
+    raw = synth.small_case(shape, seed=9)
+    dp = DenoiseParameters(radius_patchspace=(1, 1, 1), radius_searchspace=(2, 2, 2), precision="f32_fma")
+    outs = []
+    for form in (None, "column"):
+        g = IterativeNLM_GPU()
+        g.configure_device(shape, dp)
+        if form:
+            g.select_tile_form(form)
+        else:
+            assert ("paired" in g.describe()) == paired, g.describe()
+        g.set_sigma(_sigmas(shape[0])[1])
+        g.Run_GaussianNoise(1, raw)
+        outs.append(g.get_result())
+        g.free_device()
+    assert np.array_equal(outs[0], outs[1])
