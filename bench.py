@@ -156,15 +156,15 @@ def measured_peaks():
         return {}
 
 
-# DRAM traffic of one 512^3 launch of the headline filter kernel
-# (nlm_tile_f32_ws_kernel<2,2,2,raw box>: 32x8x8 CTAs of 8 consumer and 8
-# producer warps, raw box staged): dram__bytes_read.sum +
-# dram__bytes_write.sum of one 512x512x128 launch captured by ncu
-# (profiles/nlm_tile_f32_ws_p2s5_512.md gives the command), times 4: the traffic
-# is the tiles' halo boxes and the result, so it grows with the tile count.
-FILTER_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, one 512x512x128 launch of "
-                         "nlm_tile_f32_ws_kernel, x4")
-FILTER_TRAFFIC_BYTES_PER_LAUNCH = 4 * (338.045e6 + 125.709e6)
+# DRAM traffic of one 512^3 pass of the headline filter (nlm_pair_dist_kernel and
+# nlm_pair_weight_kernel at patch radius 2, search radius 5): dram__bytes_read.sum +
+# dram__bytes_write.sum over the six launches of a 256x256x96 pass captured by ncu
+# (profiles/nlm_pair_p2s5.md gives the command), scaled by the voxels. The
+# distances of half of the offsets are written once and read twice, so the
+# traffic grows with the volume (its halo share is a little smaller at 512^3).
+FILTER_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, one 256x256x96 pass of "
+                         "nlm_pair_dist_kernel and nlm_pair_weight_kernel, scaled by the voxels")
+FILTER_TRAFFIC_BYTES_PER_LAUNCH = (512.0 ** 3 / (256 * 256 * 96)) * (7.796173e9 + 13.552841e9)
 
 
 def fp32_arithmetic_peak(device: int):
