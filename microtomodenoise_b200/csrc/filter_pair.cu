@@ -220,7 +220,7 @@ __device__ __forceinline__ f32x2 square_pair(const float* c0, const float* c1, i
 // registers: a D plane is formed once, and its products serve every plane and
 // mirrored tap they belong to. Finished planes leave by TMA.
 //
-// Patch radius 1 and 2 (staged): the warp forms each D plane once over its 32
+// Patch radius 2 (staged): the warp forms each D plane once over its 32
 // columns and the patch halo, into a ring of RZ + 1 planes of its own in shared
 // memory, column-major so that a thread reads a neighbour column's 12 rows as
 // three 16-byte words (the 48-byte column pitch spreads 8 lanes over all
