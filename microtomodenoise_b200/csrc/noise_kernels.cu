@@ -377,6 +377,10 @@ __global__ void __launch_bounds__(NT, NT == kEmManyThreads ? 3 : 2)
     __shared__ float range_part[2][2 * NT / 32];
     __shared__ float range_slots[kEmMaxCluster][2];
     namespace cg = cooperative_groups;
+    // A CTA's shared memory may be written from outside once that CTA has
+    // started: every one arrives here, and the first remote store waits for all.
+    cg::cluster_group cl = cg::this_cluster();
+    cl.barrier_arrive();
     const int w = blockIdx.x / ctas;
     const unsigned rank = blockIdx.x % ctas;
     const int fs = windows[w].x, ls = windows[w].y;
@@ -413,8 +417,8 @@ __global__ void __launch_bounds__(NT, NT == kEmManyThreads ? 3 : 2)
         mn = fminf(mn, range_part[0][q]);
         mx = fmaxf(mx, range_part[1][q]);
     }
+    cl.barrier_wait();
     if (ctas > 1) {
-        cg::cluster_group cl = cg::this_cluster();
         if (tid < ctas) {
             float* dst = cl.map_shared_rank(&range_slots[rank][0], tid);
             dst[0] = mn;

@@ -32,6 +32,20 @@ def test_sigma_with_many_windows(gpu, port, n, zwindow):
     _check(port, (600, 17, 18), n, "z-adaptive", zwindow, False)
 
 
+@pytest.mark.parametrize("n,zwindow", [(60000, 140), (100000, 400)])
+def test_more_clusters_than_the_gpu_holds(gpu, n, zwindow):
+    """Hundreds of windows of two and of eight CTAs each: clusters start as others
+    end, their CTAs at different times, and every run gives the same sigma."""
+    vol = synth.small_case((600, 17, 18), seed=3)
+    dp = DenoiseParameters(noise_mode="z-adaptive", zwindow=zwindow)
+    runs = []
+    nl = NoiseLevel(n, 15, vol.shape, seed=1)
+    for _ in range(6):
+        runs.append(nl.get_noiselevel(vol, dp))
+    nl.close()
+    assert all(np.array_equal(r, runs[0]) for r in runs)
+
+
 def _check(port, shape, n, mode, zwindow, flat):
     vol = synth.small_case(shape, seed=n % 97)
     if flat:
