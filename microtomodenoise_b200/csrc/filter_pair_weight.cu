@@ -43,8 +43,13 @@ __device__ __forceinline__ bool wait_phase(uint64_t* bar, uint32_t parity) {
 // distance tiles, two offsets per stage, through a ring in shared memory by 4D
 // TMA loads (the rows of x for the first half of the offsets, of x + s for the
 // second; a copy starts on a multiple of 4 columns and is 4 columns wider than
-// the tile), and the raw tile of each z plane of offsets (the reference order
-// is z-major) through two buffers, so the consumers only wait on full barriers.
+// the tile), and the raw tile of each z plane that holds offsets (the reference
+// order is z-major) through two buffers, so the consumers only wait on full
+// barriers. Raw tiles are counted as they come, u = 0, 1, ...: u & 1 is the
+// buffer and u >> 1 its use. A stage is armed before the raw tiles of its offsets
+// are waited for: the consumers give tile u - 2 back when they enter tile u - 1,
+// which may be in the same stage (one offset per plane at the ends of a thin
+// search shape).
 //
 // What bounds it: DRAM and FP32 lanes alike. Every distance is read twice, 8
 // bytes per voxel and pair of offsets: at 256 x 256 x 96, patch radius 2, search
@@ -91,25 +96,15 @@ __global__ void __launch_bounds__(kWeightThreads, 4)
         prefetch_tmap(&tm_dist);
         prefetch_tmap(&tm_raw);
         const int zr = z % a.ring, cx = xb - a.xs, cy = yb - a.ys;
-        int g = -1, next = 0, stage = 0;
+        int g = -1, next = 0, stage = 0, u = 0, armed = 0;
         uint32_t phase = 1;  // of the empty barriers: the first round passes
         bool ok = true;
-        int s = 0;
-        for (; s < a.S; s += kStageOffsets) {
+        for (int s = 0; s < a.S && ok; s += kStageOffsets) {
             ok = wait_phase(&empty[stage], phase);
+            if (!ok) break;
             int x[kStageOffsets], y[kStageOffsets], zz[kStageOffsets];
 #pragma unroll
             for (int i = 0; i < kStageOffsets; i++) {
-                if (s + i == next) {
-                    while (s + i == next) next = a.z_start[++g + 1];
-                    const int b = g & 1;
-                    ok = ok && wait_phase(&raw_empty[b], ((g >> 1) & 1) ^ 1);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(&raw_full[b], (uint32_t)(raw_rows * RAWP * 4));
-                    // voxel xb - sxr is column px - sxr = RX of the box
-                    tma_load_3d(rawb + b * raw_bytes, &tm_raw, xb, yb - a.syr + a.py, z + g - a.szc + a.pz,
-                                &raw_full[b]);
-                }
                 const PairOffset o = a.offsets[s + i];
                 const bool first = s + i < a.H;
                 x[i] = cx + (first ? 0 : o.x);
@@ -119,12 +114,24 @@ __global__ void __launch_bounds__(kWeightThreads, 4)
                 meta[stage * kStageOffsets + i].dist = i * M::kTile + (x[i] & 3) * 4;
                 meta[stage * kStageOffsets + i].raw = (o.y * RAWP + o.x) * 4;
             }
-            if (!ok) break;
             mbar_arrive_expect_tx(&full[stage], (uint32_t)(kStageOffsets * M::TY * kDistPitch * 4));
+            armed++;
 #pragma unroll
             for (int i = 0; i < kStageOffsets; i++)
                 tma_load_4d(ring + stage * M::kStage + i * M::kTile, &tm_dist, x[i] & ~3, y[i], zz[i],
                             s + i < a.H ? s + i : a.S - 1 - s - i, &full[stage]);
+#pragma unroll
+            for (int i = 0; i < kStageOffsets; i++) {
+                if (s + i != next || !ok) continue;
+                while (s + i == next) next = a.z_start[++g + 1];
+                const int b = u & 1;
+                ok = wait_phase(&raw_empty[b], ((u >> 1) & 1) ^ 1);
+                if (!ok) continue;
+                mbar_arrive_expect_tx(&raw_full[b], (uint32_t)(raw_rows * RAWP * 4));
+                // voxel xb - sxr is column px - sxr = RX of the box
+                tma_load_3d(rawb + b * raw_bytes, &tm_raw, xb, yb - a.syr + a.py, z + g - a.szc + a.pz, &raw_full[b]);
+                u++;
+            }
             if (++stage == NS) {
                 stage = 0;
                 phase ^= 1u;
@@ -133,8 +140,8 @@ __global__ void __launch_bounds__(kWeightThreads, 4)
         if (!ok) {
             set_error(a.err, DEV_TMA_TIMEOUT);
             // let the copies in flight land before the CTA's memory goes away
-            const int n = s / kStageOffsets;
-            for (int q = max(0, n - NS); q < n; q++) mbar_wait_bounded(&full[q % NS], (q / NS) & 1);
+            for (int q = max(0, armed - NS); q < armed; q++) mbar_wait_bounded(&full[q % NS], (q / NS) & 1);
+            for (int q = max(0, u - 2); q < u; q++) mbar_wait_bounded(&raw_full[q & 1], (q >> 1) & 1);
         }
         return;
     }
@@ -150,7 +157,7 @@ __global__ void __launch_bounds__(kWeightThreads, 4)
     const unsigned char* dlane = ring + (warp * ROWS * kDistPitch + lane) * 4;
     const unsigned char* rlane = rawb + ((warp * ROWS + a.syr) * RAWP + a.px + lane) * 4;
     const unsigned char* rcur = rlane;
-    int g = -1, next = 0, stage = 0;
+    int g = -1, next = 0, stage = 0, u = 0;
     uint32_t phase = 0;
     for (int s = 0; s < a.S; s += kStageOffsets) {
         if (!wait_phase(&full[stage], phase)) {
@@ -162,13 +169,14 @@ __global__ void __launch_bounds__(kWeightThreads, 4)
             if (s + i == next) {
                 // this warp is done with the previous raw tile
                 __syncwarp();
-                if (g >= 0 && lane == 0) mbar_arrive(&raw_empty[g & 1]);
+                if (u > 0 && lane == 0) mbar_arrive(&raw_empty[(u - 1) & 1]);
                 while (s + i == next) next = a.z_start[++g + 1];
-                if (!wait_phase(&raw_full[g & 1], (g >> 1) & 1)) {
+                if (!wait_phase(&raw_full[u & 1], (u >> 1) & 1)) {
                     set_error(a.err, DEV_TMA_TIMEOUT);
                     return;
                 }
-                rcur = rlane + (g & 1) * raw_bytes;
+                rcur = rlane + (u & 1) * raw_bytes;
+                u++;
             }
             const float* dq =
                 reinterpret_cast<const float*>(dlane + stage * M::kStage + meta[stage * kStageOffsets + i].dist);

@@ -61,6 +61,23 @@ def test_paired_form_bit_exact(gpu, port, shape, pr, sr, limit):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(20, 24, 40), (42, 66, 250)])  # two and eight rows per thread
+@pytest.mark.parametrize("pr,sr,nslices", [
+    ((1, 1, 1), (1, 1, 2), 11), ((1, 1, 1), (1, 1, 5), 11), ((2, 2, 2), (1, 1, 2), 11),  # one offset in the end planes
+    ((1, 1, 1), (0, 0, 1), 11), ((1, 1, 1), (0, 0, 2), 11), ((2, 2, 2), (0, 0, 3), 11),  # no offset at z = 0
+    ((1, 1, 1), (1, 0, 3), 11), ((1, 1, 1), (0, 1, 2), 11), ((2, 2, 2), (0, 3, 2), 11), ((3, 3, 3), (3, 0, 2), 11),
+    ((1, 1, 1), (2, 2, 8), 21),
+])
+def test_thin_search_shapes_bit_exact(gpu, port, shape, pr, sr, nslices):
+    raw = synth.small_case(shape, seed=sum(sr))
+    sig = _sigmas(shape[0])
+    got, desc = _run(raw, pr, sr, sig, nslices=nslices)
+    assert "paired" in desc, desc
+    want = port.denoise_f32(raw, FilterParams(search_radius=sr, patch_radius=pr, nslices=nslices), sig, all_iters=True)
+    assert np.array_equal(got, want), f"{desc}: {np.count_nonzero(got != want)} voxels differ"
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("pr,sr", [((1, 1, 1), (3, 3, 3)), ((2, 2, 2), (4, 4, 4)), ((3, 3, 3), (2, 2, 2))])
 def test_paired_fused_form_equals_the_other_fused_kernels(gpu, pr, sr):
     raw = synth.small_case((21, 27, 50), seed=sum(pr) + sum(sr))
