@@ -352,9 +352,9 @@ int inlm::pair_filter(inlm_denoiser* d) {
                 a.tiles_z = (z1 - z + a.tz - 1) / a.tz;
                 a.splits = offset_splits(a.tiles_x * a.tiles_y * a.tiles_z, r.sms, (a.H + r.warps - 1) / r.warps);
                 CUDA_TRY(launch_pair_dist(pr[0], pr[1], pr[2], fused, r.maps, a, z, d->stream));
-                CUDA_TRY(launch_pair_weights(fused, r.maps, a, std::max(0, z - a.szc), std::min(a.nz, z1 - a.szc), r.sms,
-                                             d->stream));
-                d->launches += 2;
+                const int w0 = std::max(0, z - a.szc), w1 = std::min(a.nz, z1 - a.szc);
+                CUDA_TRY(launch_pair_weights(fused, r.maps, a, w0, w1, r.sms, d->stream));
+                d->launches += 1 + (std::max(0, w1 - w0) + kPairGridZ - 1) / kPairGridZ;
             }
         }
     return INLM_OK;

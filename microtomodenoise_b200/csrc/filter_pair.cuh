@@ -15,6 +15,7 @@ struct __align__(16) PairOffset {
     int prev;     // distance kernel: delta of s inside the staged prev box
 };
 
+constexpr int kPairGridZ = 65535;  // planes per launch of the weight kernel: the largest grid.z
 constexpr int kPairDistBox = 36;  // columns of a distance tile: 32 and the misalignment of its start
 
 struct PairArgs {

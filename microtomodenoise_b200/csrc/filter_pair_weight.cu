@@ -1,6 +1,8 @@
 // Second kernel of the paired-offset FP32 form (filter_pair.cu): weights, sums
 // and results of every voxel from the stored patch distances, all S offsets in
 // reference order (Denoiser/iternlm_cpu.cpp:758-843).
+#include <algorithm>
+
 #include "common.cuh"
 #include "filter_pair.cuh"
 #include "pair_math.cuh"
@@ -228,13 +230,18 @@ __global__ void __launch_bounds__(kWeightThreads, 4)
 template <int ROWS, int RAWP>
 cudaError_t launch_rows(bool fused, const PairMaps& m, const PairArgs& a, int z0, int z1, cudaStream_t st) {
     using M = WeightSmem<ROWS, RAWP>;
-    const dim3 grid((a.x1 - a.x0 + 31) / 32, (a.y1 - a.y0 + M::TY - 1) / M::TY, z1 - z0);
     const size_t smem = M::bytes(a.syr);
     auto kern = fused ? nlm_pair_weight_kernel<ROWS, RAWP, true> : nlm_pair_weight_kernel<ROWS, RAWP, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kWeightThreads, smem, st>>>(m.dist[ROWS != kWeightRows], m.raw[ROWS != kWeightRows], a, z0);
-    return cudaGetLastError();
+    // a plane per grid z, of which a launch takes 65535
+    for (int z = z0; z < z1; z += kPairGridZ) {
+        const dim3 grid((a.x1 - a.x0 + 31) / 32, (a.y1 - a.y0 + M::TY - 1) / M::TY, std::min(kPairGridZ, z1 - z));
+        kern<<<grid, kWeightThreads, smem, st>>>(m.dist[ROWS != kWeightRows], m.raw[ROWS != kWeightRows], a, z);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 __global__ void __launch_bounds__(256) weight_mismatch_kernel(unsigned long long* n, float nz) {

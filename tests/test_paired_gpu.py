@@ -78,6 +78,17 @@ def test_thin_search_shapes_bit_exact(gpu, port, shape, pr, sr, nslices):
 
 
 @pytest.mark.gpu
+def test_more_planes_than_a_grid_takes(gpu, port):
+    """65535 planes are the largest grid in z; a stack of 65600 is one chunk."""
+    raw = synth.small_case((65600, 5, 6), seed=4)
+    sig = _sigmas(65600)
+    got, desc = _run(raw, (1, 1, 1), (1, 1, 1), sig)
+    assert "paired" in desc, desc
+    want = port.denoise_f32(raw, FilterParams(search_radius=(1, 1, 1), patch_radius=(1, 1, 1)), sig, all_iters=True)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("pr,sr", [((1, 1, 1), (3, 3, 3)), ((2, 2, 2), (4, 4, 4)), ((3, 3, 3), (2, 2, 2))])
 def test_paired_fused_form_equals_the_other_fused_kernels(gpu, pr, sr):
     raw = synth.small_case((21, 27, 50), seed=sum(pr) + sum(sr))
