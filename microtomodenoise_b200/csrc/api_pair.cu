@@ -106,6 +106,7 @@ double warp_steps(int tiles, int splits, int sms, int warps, int H, int tz, int 
 // at z <= 0 (the reference's z-major order always is).
 int inlm::pair_configure(inlm_denoiser* d) {
     PairRun& r = d->pair;
+    pair_idle(d);  // a workspace left by a call that failed may not fit the new plan
     r.active = false;
     const Geometry& g = d->geo;
     const int* pr = g.patch_radius;
