@@ -356,9 +356,10 @@ int inlm_select_tile_form(inlm_denoiser* d, int form);
 /* Times the tiled FP32 kernel's configurations (the column form at patch
  * radius 1, CTA depth 16 with two planes per thread, CTA depth 8 with raw
  * staged in shared memory or read from global memory, depth 4, the
- * warp-specialised kernel with raw staged or from global memory) on a
- * 128x128x64 probe
- * of d's patch/search class, applies the fastest to d and caches the choice
+ * warp-specialised kernel with raw staged or from global memory) and the paired
+ * form (INLM_ERR_UNSUPPORTED where none covers d) on a 128x128x64 probe of d's
+ * patch/search class and FP32 form, applies the fastest to d (a volume with
+ * fewer tiles than the GPU has SMs keeps the paired form) and caches the choice
  * per process (and in the file named by the INLM_AUTOTUNE_CACHE environment
  * variable when set). Results do not change: every configuration rounds each
  * voxel identically. report (nullable) gets the timings. */

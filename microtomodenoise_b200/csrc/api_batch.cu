@@ -13,6 +13,7 @@
 #include <array>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -26,7 +27,7 @@ using namespace inlm;
 namespace {
 
 struct TuneKey {
-    int pr[3], sr[3], nslices, batch;
+    int pr[3], sr[3], nslices, batch;  // batch: bit 0; the fused FP32 form: bit 1
     bool operator<(const TuneKey& o) const {
         return std::lexicographical_compare(&pr[0], &pr[0] + 8, &o.pr[0], &o.pr[0] + 8);
     }
@@ -37,8 +38,17 @@ struct TuneResult {
     int tz = 8;
     bool raw_smem = true;
     bool ws = false;  // the warp-specialised 8-deep kernel
+    int paired = -1;  // the paired form: 1 faster than that, 0 slower, -1 not timed
     std::string report;
 };
+
+// The choice in words, at the end of a report.
+std::string chosen(const TuneResult& r) {
+    char line[96];
+    std::snprintf(line, sizeof line, "chosen %stz=%d%s raw_%s%s", r.paired > 0 ? "paired (without a workspace: " : "",
+                  r.tz, r.ws ? " ws" : "", r.raw_smem ? "smem" : "global", r.paired > 0 ? ")" : "");
+    return line;
+}
 
 std::mutex g_tune_mu;
 std::map<TuneKey, TuneResult> g_tune;
@@ -51,12 +61,14 @@ TuneKey tune_key(const inlm_params& p, bool batch) {
         k.sr[i] = p.search_radius[i];
     }
     k.nslices = p.nslices;
-    k.batch = batch ? 1 : 0;
+    k.batch = (batch ? 1 : 0) | (p.precision == INLM_PRECISION_F32_FMA ? 2 : 0);
     return k;
 }
 
 // Cache file (INLM_AUTOTUNE_CACHE): one line per class,
-// "pr0 pr1 pr2 sr0 sr1 sr2 nslices batch tz raw_smem".
+// "pr0 pr1 pr2 sr0 sr1 sr2 nslices batch tz flags"; flags: bit 0 raw staged, bit
+// 1 warp-specialised, bit 2 the paired form was timed too, bit 3 it was slower. A
+// line of a single volume without bit 2 is timed anew.
 void load_cache_locked() {
     if (g_tune_loaded) return;
     g_tune_loaded = true;
@@ -70,9 +82,11 @@ void load_cache_locked() {
                        &k.sr[1], &k.sr[2], &k.nslices, &k.batch, &tz, &raw) == 10) {
         TuneResult r;
         r.tz = tz;
-        r.raw_smem = (raw & 1) != 0;  // bit 0: raw staged, bit 1: warp-specialised
+        r.raw_smem = (raw & 1) != 0;
         r.ws = (raw & 2) != 0;
-        r.report = "cached";
+        if (raw & 4) r.paired = (raw & 8) ? 0 : 1;
+        if (!(k.batch & 1) && r.paired < 0) continue;
+        r.report = "cached; " + chosen(r);
         g_tune[k] = r;
     }
     std::fclose(f);
@@ -86,20 +100,23 @@ void save_cache_locked() {
     for (auto& kv : g_tune)
         std::fprintf(f, "%d %d %d %d %d %d %d %d %d %d\n", kv.first.pr[0], kv.first.pr[1],
                      kv.first.pr[2], kv.first.sr[0], kv.first.sr[1], kv.first.sr[2], kv.first.nslices,
-                     kv.first.batch, kv.second.tz, (kv.second.raw_smem ? 1 : 0) | (kv.second.ws ? 2 : 0));
+                     kv.first.batch, kv.second.tz,
+                     (kv.second.raw_smem ? 1 : 0) | (kv.second.ws ? 2 : 0) |
+                         (kv.second.paired < 0 ? 0 : kv.second.paired ? 4 : 12));
     std::fclose(f);
 }
 
-// Times every tiled configuration of a parameter class on a probe volume of
-// 128 x 128 x 64 voxels (several CTA waves on 148 SMs; the kernel's work does
-// not depend on the data) and returns the fastest. batch = true restricts the
-// candidates to the CTA depth the persistent batch kernel runs (tz 8, not the
-// warp-specialised kernel).
+// Times every tiled configuration of a parameter class, and the paired form where
+// it covers the class, on a probe volume of 128 x 128 x 64 voxels (several CTA
+// waves on 148 SMs; the kernel's work does not depend on the data) and returns
+// the fastest. batch = true restricts the candidates to the CTA depth the
+// persistent batch kernel runs (tz 8, not the warp-specialised kernel).
+constexpr int kProbe[3] = {128, 128, 64};
+
 int tune_class(const inlm_params& p0, bool batch, TuneResult* out) {
     inlm_params p = p0;
-    p.precision = INLM_PRECISION_F32;
     p.n_samples = 0;  // no noise handle
-    const int shape[3] = {128, 128, 64};
+    const int* shape = kProbe;
     inlm_denoiser* d = nullptr;
     int rc = inlm_denoiser_create(shape, &p, &d);
     if (rc) return rc;
@@ -129,6 +146,26 @@ int tune_class(const inlm_params& p0, bool batch, TuneResult* out) {
         return cleanup(fail(INLM_ERR_CUDA, "sigma upload failed"));
     rc = upload_sigma_device(d);
     if (rc) return cleanup(rc);
+    // one warm-up, two timed passes
+    auto time_passes = [&](const std::function<int()>& pass, float* ms) -> int {
+        for (int rep = 0; rep < 3; rep++) {
+            if (rep == 1) CUDA_TRY(cudaEventRecord(e0, d->stream));
+            const int prc = pass();
+            if (prc) return prc;
+        }
+        CUDA_TRY(cudaEventRecord(e1, d->stream));
+        CUDA_TRY(cudaEventSynchronize(e1));
+        CUDA_TRY(cudaEventElapsedTime(ms, e0, e1));
+        *ms *= 0.5f;
+        return INLM_OK;
+    };
+    float paired_ms = 0.f;
+    bool paired = false;
+    if (!batch) {
+        rc = pair_prepare(d, &paired);
+        if (rc == INLM_OK && paired) rc = time_passes([&] { return pair_filter(d); }, &paired_ms);
+        if (rc) return cleanup(rc);
+    }
     for (const Cand& c : cands) {
         if (batch && (c.tz != 8 || c.ws)) continue;
         bool ok = false;
@@ -137,17 +174,13 @@ int tune_class(const inlm_params& p0, bool batch, TuneResult* out) {
         if (!ok) continue;
         const int tiles_z = (shape[2] + d->tcfg.tz - 1) / d->tcfg.tz;
         float ms = 0.f;
-        for (int rep = 0; rep < 3; rep++) {  // one warm-up, two timed
-            if (rep == 1) cudaEventRecord(e0, d->stream);
-            if (launch_tile_kernel(d->tcfg, &d->tm_prev, &d->tm_raw, d->targs, tiles_z, d->stream) !=
-                cudaSuccess)
-                return cleanup(fail(INLM_ERR_CUDA, "autotune launch failed"));
-        }
-        cudaEventRecord(e1, d->stream);
-        if (cudaEventSynchronize(e1) != cudaSuccess)
-            return cleanup(fail(INLM_ERR_CUDA, "autotune timing failed"));
-        cudaEventElapsedTime(&ms, e0, e1);
-        ms *= 0.5f;
+        rc = time_passes(
+            [&]() -> int {
+                CUDA_TRY(launch_tile_kernel(d->tcfg, &d->tm_prev, &d->tm_raw, d->targs, tiles_z, d->stream));
+                return INLM_OK;
+            },
+            &ms);
+        if (rc) return cleanup(rc);
         std::snprintf(line, sizeof line, "tz=%d%s raw_%s: %.3f ms; ", c.tz, c.ws ? " ws" : "",
                       c.raw ? "smem" : "global", ms);
         res.report += line;
@@ -162,9 +195,15 @@ int tune_class(const inlm_params& p0, bool batch, TuneResult* out) {
     rc = check_device_error(d);
     if (rc) return cleanup(rc);
     if (!any) return cleanup(fail(INLM_ERR_UNSUPPORTED, "no tiled configuration for this class"));
-    std::snprintf(line, sizeof line, "chosen tz=%d%s raw_%s", res.tz, res.ws ? " ws" : "",
-                  res.raw_smem ? "smem" : "global");
-    res.report += line;
+    if (!batch) {
+        if (paired) {
+            std::snprintf(line, sizeof line, "paired: %.3f ms; ", paired_ms);
+            res.report += line;
+        }
+        // (covered, but without room for a workspace just now: not timed)
+        res.paired = paired ? paired_ms < best : d->pair.active ? -1 : 0;
+    }
+    res.report += chosen(res);
     *out = res;
     return cleanup(INLM_OK);
 }
@@ -204,6 +243,18 @@ extern "C" int inlm_autotune(inlm_denoiser* d, char* report, size_t len) {
     rc = tile_config_try(d, r.tz, r.raw_smem, &ok, r.ws);
     if (rc) return rc;
     if (!ok) return fail(INLM_ERR_STATE, "tuned configuration does not fit this volume");
+    // Volumes with fewer tiles than three quarters of the SMs keep the paired form,
+    // which shares out their offsets (the probe fills the GPU).
+    int sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
+    const long long tiles = (long long)((d->shape[0] + 31) / 32) * ((d->shape[1] + 7) / 8) * ((d->shape[2] + 7) / 8);
+    if (r.paired == 0 && 4 * tiles >= 3ll * sms) {
+        pair_release(d);
+        d->pair.active = false;
+    } else {
+        rc = pair_configure(d);
+        if (rc) return rc;
+    }
     if (report && len) std::snprintf(report, len, "%s", r.report.c_str());
     return INLM_OK;
 }
