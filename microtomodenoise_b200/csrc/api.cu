@@ -1440,7 +1440,6 @@ extern "C" int inlm_select_tile_form(inlm_denoiser* d, int form) {
     // the named forms run as named; "auto" prefers the paired form
     if (form != 0) {
         pair_release(d);
-        d->pair.active = false;
         return INLM_OK;
     }
     return pair_configure(d);

@@ -250,7 +250,6 @@ extern "C" int inlm_autotune(inlm_denoiser* d, char* report, size_t len) {
     const long long tiles = (long long)((d->shape[0] + 31) / 32) * ((d->shape[1] + 7) / 8) * ((d->shape[2] + 7) / 8);
     if (r.paired == 0 && 4 * tiles >= 3ll * sms) {
         pair_release(d);
-        d->pair.active = false;
     } else {
         rc = pair_configure(d);
         if (rc) return rc;
@@ -478,18 +477,14 @@ extern "C" int inlm_batch_create(int n, const int* shapes, const inlm_params* pa
         // 29 thousand to 1.9 million voxels. Its workspace is taken below.
         if (d->pair.active && (long long)((d->shape[0] + 31) / 32) * ((d->shape[1] + 7) / 8) *
                                       ((d->shape[2] + 7) / 8) >= sms_dev) {
-            size_t bytes = 0;
-            rc = pair_bytes(d, &bytes);
-            if (rc) return bail(rc);
-            if (bytes > 0) {
-                if (bytes > b->pair.bytes) {
-                    pair_give_back(&b->pair);
-                    if (pair_take(dev, bytes, &b->pair) != INLM_OK) b->pair = PairLoan();
-                }
-                if (b->pair.p) {
-                    paired.push_back(v);
-                    continue;  // kind stays -1
-                }
+            const size_t bytes = d->pair.bytes;
+            if (bytes > b->pair.bytes) {
+                pair_give_back(&b->pair);
+                if (pair_take(dev, bytes, &b->pair) != INLM_OK) b->pair = PairLoan();
+            }
+            if (b->pair.p) {
+                paired.push_back(v);
+                continue;  // kind stays -1
             }
         }
         // A volume whose own configuration is the column form, the 16-deep

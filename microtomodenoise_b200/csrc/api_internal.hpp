@@ -148,7 +148,6 @@ struct ProposalRun {
 // Paired-offset FP32 form (api_pair.cu): its plan and workspace.
 struct PairRun {
     bool active = false;   // filters of this handle run the paired form
-    bool planned = false;  // blocks chosen
     int bx = 0, by = 0;    // voxels per block in x and y
     int tz = 0;            // deepest tile that fits in shared memory
     int chunk = 0;         // planes per pair of launches
@@ -240,8 +239,9 @@ int upload_sigma_device(inlm_denoiser* d);
 int encode_map_f32(CUtensorMap* tm, const void* base, int rank, const long long* dims, const long long* pitch,
                    const int* box);
 // Paired-offset form: decides whether it covers the handle (after the tile
-// configuration), plans and borrows a workspace, runs one filter pass, hands the
-// workspace back (the handle's work on the GPU has ended), releases everything.
+// configuration) and plans its passes, borrows their workspace, runs one filter
+// pass, hands the workspace back (the handle's work on the GPU has ended),
+// releases everything (the form no longer runs).
 // pair_trim frees the workspace no handle has borrowed (true if there was one).
 int pair_configure(inlm_denoiser* d);
 int pair_prepare(inlm_denoiser* d, bool* ready);
@@ -250,14 +250,12 @@ void pair_idle(inlm_denoiser* d);
 void pair_release(inlm_denoiser* d);
 bool pair_trim(int device);
 // One workspace for several handles whose passes run one after another (a
-// batch): the bytes a handle's plan needs (0: the form does not run), a loan
-// for the largest, the handles bound to it.
+// batch): a loan for the largest plan, the handles bound to it.
 struct PairLoan {
     void* p = nullptr;
     size_t bytes = 0;
     int device = 0;
 };
-int pair_bytes(inlm_denoiser* d, size_t* bytes);
 int pair_take(int device, size_t bytes, PairLoan* loan);
 void pair_give_back(PairLoan* loan);
 int pair_share(inlm_denoiser* d, void* ws);

@@ -100,6 +100,87 @@ double warp_steps(int tiles, int splits, int sms, int warps, int H, int tz, int 
 
 }  // namespace
 
+// Cuts the volume into blocks (whole rows and columns where they fit) and each
+// block into z chunks, so that one chunk's distances and the search halo fit
+// the workspace. The handle runs the form where at least the smallest block fits.
+static int pair_plan(inlm_denoiser* d) {
+    PairRun& r = d->pair;
+    PairArgs& a = r.args;
+    const Geometry& g = d->geo;
+    size_t free_b = 0, total_b = 0;
+    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    size_t budget = std::min(total_b / kWorkspaceShare, (free_b + idle_bytes(d->device)) / 2);
+    if (r.limit > 0) budget = std::min(budget, r.limit);
+    const int sms = r.sms;
+    r.active = false;
+    a.dist = nullptr;  // no tensor maps yet
+    const int depth = a.nz + a.szc;  // planes whose distances are read
+    const int tz_most = r.tz, rz = g.patch_radius[2];
+    // weight kernel's time over distance kernel's (measured: 1.2, 0.6, 0.25)
+    const double weights_share = g.patch_radius[0] == 1 ? 1.2 : g.patch_radius[0] == 2 ? 0.6 : 0.25;
+    double best = 0;
+    for (int nby = 1; nby <= 32; nby++)
+        for (int nbx = 1; nbx <= 32; nbx++) {
+            const int bx = round_up((a.nx + nbx - 1) / nbx, 32), by = round_up((a.ny + nby - 1) / nby, 8);
+            if ((nbx > 1 && bx * (nbx - 1) >= a.nx) || (nby > 1 && by * (nby - 1) >= a.ny)) continue;
+            const int tiles_x = (round_up(a.sxr, 8) + std::min(bx, a.nx) + a.sxr + 31) / 32;
+            const int tiles_y = (2 * a.syr + std::min(by, a.ny) + 7) / 8;
+            const size_t plane = (size_t)tiles_x * 32 * tiles_y * 8 * a.H * 4;
+            const int ring_max = (int)std::min<size_t>(budget / plane, 1 << 20);
+            // the whole volume where it fits, else chunks of k layers of tiles
+            // of any depth down to half the deepest
+            const bool whole = depth <= ring_max;
+            for (int k = 1; k <= (whole ? 1 : 64) && (whole || (k - 1) * std::max(4, tz_most / 2) < depth); k++)
+                for (int tz = tz_most; tz >= (whole ? tz_most : std::max(4, tz_most / 2)); tz--) {
+                    const int chunk = whole ? depth : std::min(depth, k * tz), ring = whole ? depth : chunk + a.szc;
+                    if (ring > ring_max) continue;
+                    const int n_chunks = (depth + chunk - 1) / chunk;
+                    // distances: tiles of all launches (a tile of tz planes
+                    // walks tz + 2 RZ), and a third of a wave of tiles lost per
+                    // launch; weights: whole waves of CTAs (four per SM), at the
+                    // share of the time that they take
+                    const double layers = (double)((chunk + tz - 1) / tz) * n_chunks;
+                    const double walk = (double)tiles_x * tiles_y * layers / sms * (tz + 2 * rz) +
+                                        0.3 * n_chunks * (tz_most + 2 * rz);
+                    const double ctas = (double)((std::min(bx, a.nx) + 31) / 32) * ((std::min(by, a.ny) + 31) / 32) *
+                                        std::min(chunk, a.nz) / (4.0 * sms);
+                    const double cost = walk * (1.0 + weights_share * std::ceil(ctas) / ctas) * nbx * nby;
+                    if (best == 0 || cost < best) {
+                        best = cost;
+                        r.bx = bx;
+                        r.by = by;
+                        r.chunk = chunk;
+                        a.tz = tz;
+                        a.pbz = tz + 2 * rz + a.szc;
+                        a.tiles_x = tiles_x;
+                        a.tiles_y = tiles_y;
+                        a.ex = tiles_x * 32;
+                        a.ey = tiles_y * 8;
+                        a.ring = ring;
+                    }
+                }
+        }
+    if (best == 0) return INLM_OK;
+    // a volume that leaves SMs idle even with its offsets shared out: shallower
+    // tiles, whose walks are shorter
+    const int most = (a.H + r.warps - 1) / r.warps;
+    if (r.chunk == depth && a.tiles_x * a.tiles_y * ((depth + a.tz - 1) / a.tz) * most < sms) {
+        double least = 0;
+        for (int tz = tz_most; tz >= 4; tz--) {
+            const int tiles = a.tiles_x * a.tiles_y * ((depth + tz - 1) / tz);
+            const double steps = warp_steps(tiles, offset_splits(tiles, sms, most), sms, r.warps, a.H, tz, rz);
+            if (least == 0 || steps < least) {
+                least = steps;
+                a.tz = tz;
+                a.pbz = tz + 2 * rz + a.szc;
+            }
+        }
+    }
+    r.bytes = (size_t)a.H * a.ring * a.ex * a.ey * 4;
+    r.active = true;
+    return INLM_OK;
+}
+
 // Whether the paired form covers the handle's configuration: an instantiated
 // patch shape whose taps the tile kernel checked, weights that depend on
 // |x|, |y|, |z| alone, and offsets in central symmetry with the first half
@@ -158,94 +239,8 @@ int inlm::pair_configure(inlm_denoiser* d) {
     }
     if (a.tz == 0 || a.pbx > 256 || a.pby > 256 || a.pbz > 256) return INLM_OK;
     r.tz = a.tz;
-    r.planned = false;
-    r.active = true;
-    return INLM_OK;
-}
-
-// Cuts the volume into blocks (whole rows and columns where they fit) and each
-// block into z chunks, so that one chunk's distances and the search halo fit
-// the workspace; builds the offset table. Sets r.active = false where not
-// even the smallest block fits.
-static int pair_plan(inlm_denoiser* d) {
-    PairRun& r = d->pair;
-    PairArgs& a = r.args;
-    const Geometry& g = d->geo;
-    size_t free_b = 0, total_b = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    size_t budget = std::min(total_b / kWorkspaceShare, (free_b + idle_bytes(d->device)) / 2);
-    if (r.limit > 0) budget = std::min(budget, r.limit);
-    int sms = 0;
-    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
-    a.dist = nullptr;  // no tensor maps yet
-    const int depth = a.nz + a.szc;  // planes whose distances are read
-    const int tz_most = r.tz, rz = g.patch_radius[2];
-    // weight kernel's time over distance kernel's (measured: 1.2, 0.6, 0.25)
-    const double weights_share = g.patch_radius[0] == 1 ? 1.2 : g.patch_radius[0] == 2 ? 0.6 : 0.25;
-    double best = 0;
-    for (int nby = 1; nby <= 32; nby++)
-        for (int nbx = 1; nbx <= 32; nbx++) {
-            const int bx = round_up((a.nx + nbx - 1) / nbx, 32), by = round_up((a.ny + nby - 1) / nby, 8);
-            if ((nbx > 1 && bx * (nbx - 1) >= a.nx) || (nby > 1 && by * (nby - 1) >= a.ny)) continue;
-            const int tiles_x = (round_up(a.sxr, 8) + std::min(bx, a.nx) + a.sxr + 31) / 32;
-            const int tiles_y = (2 * a.syr + std::min(by, a.ny) + 7) / 8;
-            const size_t plane = (size_t)tiles_x * 32 * tiles_y * 8 * a.H * 4;
-            const int ring_max = (int)std::min<size_t>(budget / plane, 1 << 20);
-            // the whole volume where it fits, else chunks of k layers of tiles
-            // of any depth down to half the deepest
-            const bool whole = depth <= ring_max;
-            for (int k = 1; k <= (whole ? 1 : 64); k++)
-                for (int tz = tz_most; tz >= (whole ? tz_most : std::max(4, tz_most / 2)); tz--) {
-                    const int chunk = whole ? depth : std::min(depth, k * tz), ring = whole ? depth : chunk + a.szc;
-                    if (ring > ring_max) continue;
-                    const int n_chunks = (depth + chunk - 1) / chunk;
-                    // distances: tiles of all launches (a tile of tz planes
-                    // walks tz + 2 RZ), and a third of a wave of tiles lost per
-                    // launch; weights: whole waves of CTAs (four per SM), at the
-                    // share of the time that they take
-                    const double layers = (double)((chunk + tz - 1) / tz) * n_chunks;
-                    const double walk = (double)tiles_x * tiles_y * layers / sms * (tz + 2 * rz) +
-                                        0.3 * n_chunks * (tz_most + 2 * rz);
-                    const double ctas = (double)((std::min(bx, a.nx) + 31) / 32) * ((std::min(by, a.ny) + 31) / 32) *
-                                        std::min(chunk, a.nz) / (4.0 * sms);
-                    const double cost = walk * (1.0 + weights_share * std::ceil(ctas) / ctas) * nbx * nby;
-                    if (best == 0 || cost < best) {
-                        best = cost;
-                        r.bx = bx;
-                        r.by = by;
-                        r.chunk = chunk;
-                        a.tz = tz;
-                        a.pbz = tz + 2 * rz + a.szc;
-                        a.tiles_x = tiles_x;
-                        a.tiles_y = tiles_y;
-                        a.ex = tiles_x * 32;
-                        a.ey = tiles_y * 8;
-                        a.ring = ring;
-                    }
-                }
-        }
-    if (best == 0) {
-        r.active = false;
-        return INLM_OK;
-    }
-    r.sms = sms;
-    r.warps = pair_kernel_warps(g.patch_radius[0]);
-    // a volume that leaves SMs idle even with its offsets shared out: shallower
-    // tiles, whose walks are shorter
-    const int most = (a.H + r.warps - 1) / r.warps;
-    if (r.chunk == depth && a.tiles_x * a.tiles_y * ((depth + a.tz - 1) / a.tz) * most < sms) {
-        double least = 0;
-        for (int tz = tz_most; tz >= 4; tz--) {
-            const int tiles = a.tiles_x * a.tiles_y * ((depth + tz - 1) / tz);
-            const double steps = warp_steps(tiles, offset_splits(tiles, sms, most), sms, r.warps, a.H, tz, rz);
-            if (least == 0 || steps < least) {
-                least = steps;
-                a.tz = tz;
-                a.pbz = tz + 2 * rz + a.szc;
-            }
-        }
-    }
-    const int S = a.S;
+    CUDA_TRY(cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, d->device));
+    r.warps = pair_kernel_warps(pr[0]);
     std::vector<PairOffset> t(S);
     for (int s = 0; s < S; s++) {
         const Offset3& o = g.search[s];
@@ -257,7 +252,6 @@ static int pair_plan(inlm_denoiser* d) {
     std::vector<int> zs(2 * a.szc + 2, S);  // first offset of every z
     for (int s = S - 1; s >= 0; s--) zs[g.search[s].z + a.szc] = s;
     for (int i = 2 * a.szc; i >= 0; i--) zs[i] = std::min(zs[i], zs[i + 1]);
-    r.bytes = (size_t)a.H * a.ring * a.ex * a.ey * 4;
     CUDA_TRY(r.offsets.ensure(S * sizeof(PairOffset)));
     CUDA_TRY(r.z_start.ensure(zs.size() * sizeof(int)));
     CUDA_TRY(cudaMemcpyAsync(r.offsets.p, t.data(), S * sizeof(PairOffset), cudaMemcpyHostToDevice, d->stream));
@@ -272,8 +266,7 @@ static int pair_plan(inlm_denoiser* d) {
     a.out = d->d_next;
     a.mult = d->d_mult;
     a.err = d->d_err;
-    r.planned = true;
-    return INLM_OK;
+    return pair_plan(d);
 }
 
 // Points the handle's kernels at a workspace of at least r.bytes.
@@ -301,7 +294,8 @@ static int pair_bind(inlm_denoiser* d, void* ws) {
 }
 
 // Borrows a workspace for the handle's next passes; *ok = false where there is
-// no room for one.
+// no room for one. Where memory has become scarce since the handle was configured,
+// the passes are planned anew for what is left.
 static int pair_borrow(inlm_denoiser* d, bool* ok) {
     PairRun& r = d->pair;
     *ok = true;
@@ -310,7 +304,16 @@ static int pair_borrow(inlm_denoiser* d, bool* ok) {
         count_user(d->device, 1);
         r.user = true;
     }
-    if (borrow(d->device, r.bytes, &r.dist, &r.dist_bytes) != cudaSuccess) {
+    bool got = borrow(d->device, r.bytes, &r.dist, &r.dist_bytes) == cudaSuccess;
+    if (!got) {
+        cudaGetLastError();
+        const size_t wanted = r.bytes;
+        const int rc = pair_plan(d);
+        if (rc) return rc;
+        got = r.active && r.bytes < wanted && borrow(d->device, r.bytes, &r.dist, &r.dist_bytes) == cudaSuccess;
+        r.active = true;  // a later call may find room again
+    }
+    if (!got) {
         cudaGetLastError();
         r.dist = nullptr;
         *ok = false;
@@ -319,16 +322,11 @@ static int pair_borrow(inlm_denoiser* d, bool* ok) {
     return pair_bind(d, r.dist);
 }
 
-// Plans the handle's passes and borrows their workspace; *ready = false when the
-// form does not run here.
+// Borrows the workspace of the handle's passes; *ready = false when the form does
+// not run here.
 int inlm::pair_prepare(inlm_denoiser* d, bool* ready) {
-    PairRun& r = d->pair;
     *ready = false;
-    if (r.active && !r.planned) {
-        const int rc = pair_plan(d);
-        if (rc) return rc;
-    }
-    return r.active ? pair_borrow(d, ready) : INLM_OK;
+    return d->pair.active ? pair_borrow(d, ready) : INLM_OK;
 }
 
 // Enqueues one filter pass.
@@ -358,17 +356,6 @@ int inlm::pair_filter(inlm_denoiser* d) {
                 d->launches += 1 + (std::max(0, w1 - w0) + kPairGridZ - 1) / kPairGridZ;
             }
         }
-    return INLM_OK;
-}
-
-int inlm::pair_bytes(inlm_denoiser* d, size_t* bytes) {
-    PairRun& r = d->pair;
-    *bytes = 0;
-    if (r.active && !r.planned) {
-        const int rc = pair_plan(d);
-        if (rc) return rc;
-    }
-    if (r.active) *bytes = r.bytes;
     return INLM_OK;
 }
 
@@ -418,7 +405,7 @@ void inlm::pair_release(inlm_denoiser* d) {
     r.user = false;
     r.offsets.release();
     r.z_start.release();
-    r.planned = false;
+    r.active = false;
 }
 
 extern "C" int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes) {
@@ -426,9 +413,9 @@ extern "C" int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes) {
     if (!d->pair.active) return fail(INLM_ERR_UNSUPPORTED, "the paired form does not run on this handle");
     CUDA_TRY(cudaSetDevice(d->device));
     CUDA_TRY(cudaStreamSynchronize(d->stream));
-    pair_release(d);
+    pair_idle(d);
     d->pair.limit = (size_t)bytes;
-    return INLM_OK;
+    return pair_plan(d);
 }
 
 extern "C" int inlm_debug_weight_mismatches(int64_t* n) {

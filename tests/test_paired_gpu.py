@@ -124,6 +124,39 @@ def test_paired_form_without_room_for_its_workspace(gpu, port):
 
 
 @pytest.mark.gpu
+def test_first_pass_allocates_its_workspace_and_nothing_else(gpu, port):
+    """Plan and tables are made when the handle is configured: a first pass takes
+    a workspace (which may fail: the single-pass kernel runs) and a second nothing."""
+    L = _lib.load()
+
+    def live():
+        n = C.c_int64(0)
+        _lib.check(L.inlm_debug_live_allocations(C.byref(n)), "live allocations")
+        return n.value
+
+    raw = synth.small_case((20, 24, 40), seed=5)
+    sig = _sigmas(20)
+    want = port.denoise_f32(raw, FilterParams(search_radius=(3, 3, 3), patch_radius=(2, 2, 2)), sig, all_iters=True)
+    g = IterativeNLM_GPU()
+    g.configure_device(raw.shape, DenoiseParameters(radius_patchspace=(2, 2, 2), radius_searchspace=(3, 3, 3)))
+    before = live()
+    g.set_sigma(sig[0])
+    L.inlm_debug_fail_allocation(0)
+    g.Run_GaussianNoise(1, raw)
+    L.inlm_debug_fail_allocation(-1)
+    assert np.array_equal(g.get_result(), want[0]) and live() == before
+    g.Run_GaussianNoise(1, raw)
+    assert np.array_equal(g.get_result(), want[0]) and live() == before + 1
+    g.set_sigma(sig[1])
+    L.inlm_debug_fail_allocation(0)  # (nothing is allocated, so nothing fails)
+    g.Run_GaussianNoise(2)
+    L.inlm_debug_fail_allocation(-1)
+    assert np.array_equal(g.get_result(), want[1]) and live() == before + 1
+    assert "paired" in g.describe()
+    g.free_device()
+
+
+@pytest.mark.gpu
 def test_paired_handles_take_turns_on_one_workspace(gpu):
     L = _lib.load()
     live = C.c_int64(0)
