@@ -175,12 +175,18 @@ int inlm_debug_live_allocations(int64_t* n);
 int inlm_debug_wait_expiry(inlm_denoiser* d, int64_t cycles);
 /* Test hooks of the paired-offset FP32 form. inlm_debug_pair_workspace bounds
  * the handle's workspace to `bytes` (0: the default), so that small volumes are
- * cut into blocks and z chunks as large ones are; INLM_ERR_UNSUPPORTED where
- * the form does not run. inlm_debug_weight_mismatches compares, on the current
+ * cut into blocks and z chunks as large ones are, faster than the single-pass
+ * kernel or not; with -bytes the form runs only where it is faster, as by itself;
+ * INLM_ERR_UNSUPPORTED where the form does not cover the handle. inlm_debug_pair_plan gives, for
+ * a workspace of `bytes` on a B200 (no device needed), whether the form runs, the
+ * time of its plan and that of the whole volume in one chunk (the same unit), the
+ * plan's bytes, its block's x and y, planes per chunk and per tile.
+ * inlm_debug_weight_mismatches compares, on the current
  * device, the form's weight step with the other kernels' for every float x in
  * [-3.6, -0] and stores how many differ. */
 int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes);
 int inlm_debug_weight_mismatches(int64_t* n);
+int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, int64_t bytes, double out[8]);
 
 /* Number of kernels this handle has launched since creation. */
 int inlm_kernel_launches(inlm_denoiser* d, uint64_t* count);

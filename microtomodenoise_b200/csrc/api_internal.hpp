@@ -157,6 +157,7 @@ struct PairRun {
     int sms = 0;
     inlm::DevBuf offsets, z_start;
     size_t limit = 0;       // bound on the workspace set by a test (0: none)
+    bool forced = false;    // the form runs within it whether or not that is faster
     size_t bytes = 0;       // workspace the plan needs
     void* dist = nullptr;   // borrowed workspace (pair_idle hands it back)
     size_t dist_bytes = 0;

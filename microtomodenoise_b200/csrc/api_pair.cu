@@ -1,5 +1,7 @@
 // Host side of the paired-offset FP32 form (filter_pair.cu): when it applies,
 // the workspace and how a volume is cut into blocks and z chunks that fit it.
+#include <cmath>
+#include <cstdlib>
 #include <mutex>
 
 #include "api_internal.hpp"
@@ -98,27 +100,26 @@ double warp_steps(int tiles, int splits, int sms, int warps, int H, int tz, int 
     return rounds * ((tiles * (long long)splits + sms - 1) / sms);
 }
 
-}  // namespace
+// A volume cut into blocks (whole rows and columns where they fit) and each block
+// into z chunks, so that one chunk's distances and the search halo fit a
+// workspace.
+struct Plan {
+    int bx = 0, by = 0;          // voxels per block in x and y
+    int chunk = 0;               // planes per pair of launches
+    int tz = 0;                  // planes per tile
+    int tiles_x = 0, tiles_y = 0;
+    int ring = 0;                // workspace planes per offset
+    double cost = 0;             // 0: not even the smallest block fits
+    size_t bytes(int H) const { return (size_t)H * ring * tiles_x * 32 * tiles_y * 8 * 4; }
+};
 
-// Cuts the volume into blocks (whole rows and columns where they fit) and each
-// block into z chunks, so that one chunk's distances and the search halo fit
-// the workspace. The handle runs the form where at least the smallest block fits.
-static int pair_plan(inlm_denoiser* d) {
-    PairRun& r = d->pair;
-    PairArgs& a = r.args;
-    const Geometry& g = d->geo;
-    size_t free_b = 0, total_b = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    size_t budget = std::min(total_b / kWorkspaceShare, (free_b + idle_bytes(d->device)) / 2);
-    if (r.limit > 0) budget = std::min(budget, r.limit);
-    const int sms = r.sms;
-    r.active = false;
-    a.dist = nullptr;  // no tensor maps yet
+// The cheapest plan for a workspace of `budget` bytes; a.tz is the deepest tile.
+Plan plan_blocks(const PairArgs& a, const int* pr, int sms, int warps, size_t budget) {
+    Plan best;
     const int depth = a.nz + a.szc;  // planes whose distances are read
-    const int tz_most = r.tz, rz = g.patch_radius[2];
+    const int tz_most = a.tz, rz = pr[2];
     // weight kernel's time over distance kernel's (measured: 1.2, 0.6, 0.25)
-    const double weights_share = g.patch_radius[0] == 1 ? 1.2 : g.patch_radius[0] == 2 ? 0.6 : 0.25;
-    double best = 0;
+    const double weights_share = pr[0] == 1 ? 1.2 : pr[0] == 2 ? 0.6 : 0.25;
     for (int nby = 1; nby <= 32; nby++)
         for (int nbx = 1; nbx <= 32; nbx++) {
             const int bx = round_up((a.nx + nbx - 1) / nbx, 32), by = round_up((a.ny + nby - 1) / nby, 8);
@@ -145,38 +146,110 @@ static int pair_plan(inlm_denoiser* d) {
                     const double ctas = (double)((std::min(bx, a.nx) + 31) / 32) * ((std::min(by, a.ny) + 31) / 32) *
                                         std::min(chunk, a.nz) / (4.0 * sms);
                     const double cost = walk * (1.0 + weights_share * std::ceil(ctas) / ctas) * nbx * nby;
-                    if (best == 0 || cost < best) {
-                        best = cost;
-                        r.bx = bx;
-                        r.by = by;
-                        r.chunk = chunk;
-                        a.tz = tz;
-                        a.pbz = tz + 2 * rz + a.szc;
-                        a.tiles_x = tiles_x;
-                        a.tiles_y = tiles_y;
-                        a.ex = tiles_x * 32;
-                        a.ey = tiles_y * 8;
-                        a.ring = ring;
-                    }
+                    if (best.cost == 0 || cost < best.cost) best = Plan{bx, by, chunk, tz, tiles_x, tiles_y, ring, cost};
                 }
         }
-    if (best == 0) return INLM_OK;
     // a volume that leaves SMs idle even with its offsets shared out: shallower
     // tiles, whose walks are shorter
-    const int most = (a.H + r.warps - 1) / r.warps;
-    if (r.chunk == depth && a.tiles_x * a.tiles_y * ((depth + a.tz - 1) / a.tz) * most < sms) {
+    const int most = (a.H + warps - 1) / warps;
+    if (best.cost > 0 && best.chunk == depth &&
+        best.tiles_x * best.tiles_y * ((depth + best.tz - 1) / best.tz) * most < sms) {
         double least = 0;
         for (int tz = tz_most; tz >= 4; tz--) {
-            const int tiles = a.tiles_x * a.tiles_y * ((depth + tz - 1) / tz);
-            const double steps = warp_steps(tiles, offset_splits(tiles, sms, most), sms, r.warps, a.H, tz, rz);
+            const int tiles = best.tiles_x * best.tiles_y * ((depth + tz - 1) / tz);
+            const double steps = warp_steps(tiles, offset_splits(tiles, sms, most), sms, warps, a.H, tz, rz);
             if (least == 0 || steps < least) {
                 least = steps;
-                a.tz = tz;
-                a.pbz = tz + 2 * rz + a.szc;
+                best.tz = tz;
             }
         }
     }
-    r.bytes = (size_t)a.H * a.ring * a.ex * a.ey * 4;
+    return best;
+}
+
+// A plan's time in units of a plane step of a tile on one SM. Unlike the cost that
+// plans are chosen by, it counts the weight kernel's CTAs in the rows per thread
+// that a chunk gets: within 15 % of the measured ratio up to half again the time of
+// the whole volume in one chunk, above it beyond.
+double plan_time(const PairArgs& a, const int* pr, int sms, const Plan& p) {
+    const int depth = a.nz + a.szc, rz = pr[2], wx = std::min(p.bx, a.nx), wy = std::min(p.by, a.ny);
+    const double weights_share = pr[0] == 1 ? 1.2 : pr[0] == 2 ? 0.6 : 0.25;
+    const int blocks = (a.nx + p.bx - 1) / p.bx * ((a.ny + p.by - 1) / p.by), n_chunks = (depth + p.chunk - 1) / p.chunk;
+    const double layers = (double)((p.chunk + p.tz - 1) / p.tz) * n_chunks;
+    const double dist = (double)p.tiles_x * p.tiles_y * layers / sms * (p.tz + 2 * rz) + 0.3 * n_chunks * (a.tz + 2 * rz);
+    const int columns = (wx + 31) / 32, planes = std::min(p.chunk, a.nz);
+    const int rows = pair_weight_rows(pair_weight_small((long long)columns * ((wy + 7) / 8) * planes, sms));
+    const double ctas = (double)columns * ((wy + rows - 1) / rows) * planes / (4.0 * sms);
+    const double weights = weights_share * columns * ((wy + 7) / 8) * a.nz / sms * std::ceil(ctas) / ctas;
+    return (dist + weights) * blocks;
+}
+
+// Whether a plan is worth running: the single-pass kernels take kSingle times as
+// long as the whole volume in one chunk, so a plan that is cut up further is slower
+// than they are. Measured at 256^3 as workspace: paired (single-pass), ms. Patch
+// radius 1, search radius 10, 22 GB: 92.9, 16: 96.8, 8: 113.7, 4: 130.9, 2: 149, 1:
+// 296 (102.6); search radius 5, 22 GB: 13.9, 2: 16.1, 1: 20.0 (17.1). Patch radius
+// 2, search radius 5, 22 GB: 19.7, 1: 27.3, 0.5: 30.8, 0.25: 42.5 (36.1). Patch
+// radius 3, search radius 7, 22 GB: 112, 2: 138, 1: 167, 0.5: 221, 0.25: 396 (262).
+bool plan_pays(const PairArgs& a, const int* pr, int sms, int warps, const Plan& p) {
+    const double kSingle = pr[0] == 1 ? 1.18 : pr[0] == 2 ? 1.85 : 2.3;
+    return p.cost > 0 && plan_time(a, pr, sms, p) <= kSingle * plan_time(a, pr, sms, plan_blocks(a, pr, sms, warps, SIZE_MAX));
+}
+
+// Extents of the form's kernels for a volume: false where they do not cover it.
+// a->tz is the deepest tile whose box fits beside the warps' buffers.
+bool pair_extents(const Geometry& g, const int shape[3], int nslices, size_t smem_max, PairArgs* a) {
+    const int* pr = g.patch_radius;
+    *a = PairArgs{};
+    a->nx = shape[0];
+    a->ny = shape[1];
+    a->nz = shape[2];
+    a->px = g.pad[0];
+    a->py = g.pad[1];
+    a->pz = g.pad[2];
+    a->sxr = g.search_radius[0];
+    a->syr = g.search_radius[1];
+    a->szc = std::min(nslices / 2, g.search_radius[2]);
+    a->S = (int)g.search.size();
+    a->H = a->S / 2;
+    a->pbx = pair_box_pitch(a->px);
+    if (a->pbx == 0) return false;
+    a->pby = 8 + 2 * a->py;
+    for (int tz = 24; tz >= 4 && a->tz == 0; tz--) {
+        a->pbz = tz + 2 * pr[2] + a->szc;
+        if (pair_smem_bytes(pr[0], pr[2], *a) <= smem_max) a->tz = tz;
+    }
+    return a->tz > 0 && a->pbx <= 256 && a->pby <= 256 && a->pbz <= 256;
+}
+
+}  // namespace
+
+// Plans the handle's passes for the memory there is; the handle runs the form where
+// the plan is faster than the single-pass kernel.
+static int pair_plan(inlm_denoiser* d) {
+    PairRun& r = d->pair;
+    PairArgs& a = r.args;
+    const int* pr = d->geo.patch_radius;
+    size_t free_b = 0, total_b = 0;
+    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    size_t budget = std::min(total_b / kWorkspaceShare, (free_b + idle_bytes(d->device)) / 2);
+    if (r.limit > 0) budget = std::min(budget, r.limit);
+    a.tz = r.tz;
+    const Plan plan = plan_blocks(a, pr, r.sms, r.warps, budget);
+    r.active = false;
+    a.dist = nullptr;  // no tensor maps yet
+    if (plan.cost == 0 || (!r.forced && !plan_pays(a, pr, r.sms, r.warps, plan))) return INLM_OK;
+    r.bx = plan.bx;
+    r.by = plan.by;
+    r.chunk = plan.chunk;
+    a.tz = plan.tz;
+    a.pbz = a.tz + 2 * pr[2] + a.szc;
+    a.tiles_x = plan.tiles_x;
+    a.tiles_y = plan.tiles_y;
+    a.ex = plan.tiles_x * 32;
+    a.ey = plan.tiles_y * 8;
+    a.ring = plan.ring;
+    r.bytes = plan.bytes(a.H);
     r.active = true;
     return INLM_OK;
 }
@@ -213,31 +286,10 @@ int inlm::pair_configure(inlm_denoiser* d) {
         if (4 * ctas >= 3ll * sms) return INLM_OK;
     }
     PairArgs& a = r.args;
-    a = PairArgs{};
-    a.nx = d->shape[0];
-    a.ny = d->shape[1];
-    a.nz = d->shape[2];
-    a.px = g.pad[0];
-    a.py = g.pad[1];
-    a.pz = g.pad[2];
-    a.sxr = g.search_radius[0];
-    a.syr = g.search_radius[1];
-    a.szc = std::min(d->p.nslices / 2, g.search_radius[2]);
-    a.S = S;
-    a.H = S / 2;
-    a.pbx = pair_box_pitch(a.px);
-    if (a.pbx == 0) return INLM_OK;
-    a.pby = 8 + 2 * a.py;
-    for (int t = 0; t < (int)g.taps.size(); t++) a.w[t] = g.weights[t];
-    // the deepest tile whose box fits beside the warps' buffers
     int smem_max = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
-    a.tz = 0;
-    for (int tz = 24; tz >= 4 && a.tz == 0; tz--) {
-        a.pbz = tz + 2 * pr[2] + a.szc;
-        if (pair_smem_bytes(pr[0], pr[2], a) <= (size_t)smem_max) a.tz = tz;
-    }
-    if (a.tz == 0 || a.pbx > 256 || a.pby > 256 || a.pbz > 256) return INLM_OK;
+    if (!pair_extents(g, d->shape, d->p.nslices, smem_max, &a)) return INLM_OK;
+    for (int t = 0; t < (int)g.taps.size(); t++) a.w[t] = g.weights[t];
     r.tz = a.tz;
     CUDA_TRY(cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, d->device));
     r.warps = pair_kernel_warps(pr[0]);
@@ -409,13 +461,31 @@ void inlm::pair_release(inlm_denoiser* d) {
 }
 
 extern "C" int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes) {
-    if (!d || bytes < 0) return fail(INLM_ERR_ARG, "bad argument");
-    if (!d->pair.active) return fail(INLM_ERR_UNSUPPORTED, "the paired form does not run on this handle");
+    if (!d) return fail(INLM_ERR_ARG, "null handle");
+    if (!d->pair.offsets.p) return fail(INLM_ERR_UNSUPPORTED, "the paired form does not cover this handle");
     CUDA_TRY(cudaSetDevice(d->device));
     CUDA_TRY(cudaStreamSynchronize(d->stream));
     pair_idle(d);
-    d->pair.limit = (size_t)bytes;
+    d->pair.limit = (size_t)std::llabs(bytes);
+    d->pair.forced = bytes > 0;
     return pair_plan(d);
+}
+
+extern "C" int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, int64_t bytes, double out[8]) {
+    if (!shape || !p || !out || bytes < 0) return fail(INLM_ERR_ARG, "bad argument");
+    const int* pr = p->patch_radius;
+    if (!pair_kernel_available(pr[0], pr[1], pr[2])) return fail(INLM_ERR_UNSUPPORTED, "no kernels of this patch shape");
+    const int pz = std::min(p->nslices / 2, p->search_radius[2]) + pr[2];
+    const Geometry g = make_geometry(p->search_radius, pr, p->nslices, p->z_anisotropy, p->weight_table, shape[2] + 2 * pz);
+    PairArgs a;
+    if (!pair_extents(g, shape, p->nslices, 227 * 1024, &a)) return fail(INLM_ERR_UNSUPPORTED, "the box does not fit");
+    const Plan most = plan_blocks(a, pr, 148, pair_kernel_warps(pr[0]), SIZE_MAX);
+    const Plan plan = plan_blocks(a, pr, 148, pair_kernel_warps(pr[0]), (size_t)bytes);
+    const double runs = plan_pays(a, pr, 148, pair_kernel_warps(pr[0]), plan) ? 1.0 : 0.0;
+    const double v[8] = {runs, plan.cost > 0 ? plan_time(a, pr, 148, plan) : 0.0, plan_time(a, pr, 148, most), (double)plan.bytes(a.H), (double)plan.bx,
+                         (double)plan.by, (double)plan.chunk, (double)plan.tz};
+    std::copy(v, v + 8, out);
+    return INLM_OK;
 }
 
 extern "C" int inlm_debug_weight_mismatches(int64_t* n) {

@@ -65,6 +65,7 @@ struct PairMaps {
 cudaError_t launch_pair_dist(int rx, int ry, int rz, bool fused, const PairMaps& m, const PairArgs& a, int z0,
                              cudaStream_t st);
 int pair_weight_rows(int i);  // rows per CTA: i 0 (8 rows per thread), 1 (2 rows)
+int pair_weight_small(long long warps, int sms);  // that i, for a launch of so many warps of 32 x 8 voxels
 // Weights, sums and results of the planes [z0, z1) from the ring.
 cudaError_t launch_pair_weights(bool fused, const PairMaps& m, const PairArgs& a, int z0, int z1, int sms,
                                 cudaStream_t st);

@@ -266,12 +266,13 @@ cudaError_t launch_weight_mismatches(unsigned long long* n, float neg0, cudaStre
 
 int pair_weight_rows(int i) { return kWeightWarps * (i ? kWeightRowsSmall : kWeightRows); }
 
+// 8 rows per thread where that still gives every SM its warps, else 2
+int pair_weight_small(long long warps, int sms) { return warps < 16ll * sms; }
+
 cudaError_t launch_pair_weights(bool fused, const PairMaps& m, const PairArgs& a, int z0, int z1, int sms,
                                 cudaStream_t st) {
     if (z1 <= z0) return cudaSuccess;
-    // 8 rows per thread where that still gives every SM its warps, else 2
-    const long long warps = (long long)((a.x1 - a.x0 + 31) / 32) * ((a.y1 - a.y0 + 7) / 8) * (z1 - z0);
-    const bool big = warps >= 16ll * sms;
+    const bool big = !pair_weight_small((long long)((a.x1 - a.x0 + 31) / 32) * ((a.y1 - a.y0 + 7) / 8) * (z1 - z0), sms);
 #define X(PITCH)                                                                       \
     if (a.pbx == PITCH)                                                                 \
         return big ? launch_rows<kWeightRows, PITCH>(fused, m, a, z0, z1, st)         \

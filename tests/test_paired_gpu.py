@@ -124,6 +124,19 @@ def test_paired_form_without_room_for_its_workspace(gpu, port):
 
 
 @pytest.mark.gpu
+def test_a_plan_slower_than_the_single_pass_kernel_does_not_run(gpu, port):
+    raw = synth.small_case((40, 64, 96), seed=7)
+    sig = _sigmas(40)
+    want = port.denoise_f32(raw, FilterParams(search_radius=(5, 5, 5), patch_radius=(1, 1, 1)), sig, all_iters=True)
+    got, desc = _run(raw, (1, 1, 1), (5, 5, 5), sig, limit=-32 * MB)
+    assert desc.startswith("nlm_column_f32<"), desc
+    assert np.array_equal(got, want)
+    got, desc = _run(raw, (1, 1, 1), (5, 5, 5), sig, limit=32 * MB)
+    assert "paired" in desc, desc
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.gpu
 def test_first_pass_allocates_its_workspace_and_nothing_else(gpu, port):
     """Plan and tables are made when the handle is configured: a first pass takes
     a workspace (which may fail: the single-pass kernel runs) and a second nothing."""
