@@ -13,6 +13,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -176,6 +178,21 @@ int inlm::encode_map_f32(CUtensorMap* tm, const void* base, int rank, const long
                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(INLM_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return INLM_OK;
+}
+
+// ---------------- kernel attributes ----------------
+
+cudaError_t inlm::allow_shared_memory(const void* kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> largest;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& most = largest[{kernel, device}];
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(most, bytes));
+    if (e == cudaSuccess) most = std::max(most, bytes);
+    return e;
 }
 
 // ---------------- noise handle ----------------

@@ -10,6 +10,7 @@
 #include <utility>
 
 #include "color_kernels.cuh"
+#include "common.cuh"
 #include "geometry.hpp"
 
 namespace inlm {
@@ -305,7 +306,7 @@ int rgb_tap_order(int r, int* dxdy, int max_taps) {
 template <typename K>
 static cudaError_t launch_with(K kern, const RgbArgs& a, cudaStream_t st) {
     const size_t smem = rgb_smem_bytes(a);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nx + kRgbTX - 1) / kRgbTX, (a.ny + kRgbTY - 1) / kRgbTY);
     kern<<<grid, dim3(kRgbTX, kRgbTY), smem, st>>>(a);

@@ -8,6 +8,15 @@
 
 namespace inlm {
 
+// Allows a kernel's launches on the current device `bytes` of dynamic shared
+// memory. The limit is only ever raised: another thread may be about to launch
+// the same kernel with more than this handle's configuration takes.
+cudaError_t allow_shared_memory(const void* kernel, size_t bytes);
+template <class... A>
+cudaError_t allow_shared_memory(void (*kernel)(A...), size_t bytes) {
+    return allow_shared_memory(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Device error codes written to the per-handle error word.
 enum DeviceError : int {
     DEV_OK = 0,

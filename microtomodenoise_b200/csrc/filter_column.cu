@@ -288,7 +288,7 @@ template <int RX, int RY, int RZ, int TZ>
 cudaError_t launch_column(const CUtensorMap* tm, const TileArgs& a, int tiles_z, size_t smem, bool fused,
                           cudaStream_t st) {
     auto kern = fused ? nlm_column_f32_kernel<RX, RY, RZ, TZ, true> : nlm_column_f32_kernel<RX, RY, RZ, TZ, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.tiles_x, a.tiles_y, tiles_z);
     kern<<<grid, 32 * TZ, smem, st>>>(*tm, a);
@@ -494,7 +494,7 @@ template <int RX, int RY, int RZ, int TZ>
 cudaError_t launch_column_fast(const CUtensorMap* tm, const FastArgs& a, int tiles_z, size_t smem, bool d_half,
                                cudaStream_t st) {
     auto kern = d_half ? nlm_column_fast_kernel<RX, RY, RZ, TZ, true> : nlm_column_fast_kernel<RX, RY, RZ, TZ, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.tiles_x, a.tiles_y, tiles_z);
     kern<<<grid, 32 * TZ, smem, st>>>(*tm, a);

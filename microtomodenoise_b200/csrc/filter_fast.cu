@@ -572,7 +572,7 @@ static cudaError_t fast_launch_inst(const CUtensorMap* tmp, const FastArgs& a, i
         else
             return cudaErrorInvalidConfiguration;
     }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.tiles_x, a.tiles_y, tiles_z);
     kern<<<grid, TX * TZ * 8 / FastThreads<TX>::VPT, smem, st>>>(*tmp, a);

@@ -1017,7 +1017,7 @@ template <int RX, int RY, int RZ, bool SLAB>
 static cudaError_t launch_z2(const CUtensorMap* tmp, const TileArgs& a, int tiles_z, size_t smem,
                              cudaStream_t st) {
     auto kern = nlm_tile_f32_z2_kernel<RX, RY, RZ, SLAB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.tiles_x, a.tiles_y, tiles_z);
     kern<<<grid, 256, smem, st>>>(*tmp, a);
@@ -1029,7 +1029,7 @@ static cudaError_t launch_inst(const CUtensorMap* tmp, const CUtensorMap* tmr, c
                                int tiles_z, size_t smem, cudaStream_t st) {
     (void)tmr;
     auto kern = nlm_tile_f32_kernel<RX, RY, RZ, TZ, RAW_SMEM, FUSED, SLAB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.tiles_x, a.tiles_y, tiles_z);
     kern<<<grid, 32 * TZ, smem, st>>>(*tmp, a);
@@ -1049,8 +1049,7 @@ int batch_kind(const TileConfig& c) {
 
 template <int R, bool RAW, bool SLAB = false>
 static cudaError_t batch_setup_r(size_t smem, int* ctas_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(nlm_batch_f32_kernel<R, RAW, SLAB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(nlm_batch_f32_kernel<R, RAW, SLAB>, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, nlm_batch_f32_kernel<R, RAW, SLAB>,
                                                          256, smem);
@@ -1133,7 +1132,7 @@ static cudaError_t launch_ws(const CUtensorMap* tmp, const TileArgs& a, int tile
                                   : nlm_tile_f32_ws_kernel<RX, RY, RZ, false, true>)
                       : (raw_smem ? nlm_tile_f32_ws_kernel<RX, RY, RZ, true, false>
                                   : nlm_tile_f32_ws_kernel<RX, RY, RZ, false, false>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.tiles_x, a.tiles_y, tiles_z);
     kern<<<grid, WsThreads<RX>::N, smem, st>>>(*tmp, a);

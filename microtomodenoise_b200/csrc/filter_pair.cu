@@ -448,7 +448,7 @@ template <int RX, int RY, int RZ, int PBX>
 cudaError_t launch_dist_pitch(bool fused, const PairMaps& m, const PairArgs& a, int z0, cudaStream_t st) {
     const size_t smem = pair_smem_bytes(RX, RZ, a);
     auto kern = fused ? nlm_pair_dist_kernel<RX, RY, RZ, PBX, true> : nlm_pair_dist_kernel<RX, RY, RZ, PBX, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<a.tiles_x * a.tiles_y * a.tiles_z * a.splits, 32 * PairSmem<RX, RZ>::kWarps, smem, st>>>(m.prev, m.out, a, z0);
     return cudaGetLastError();

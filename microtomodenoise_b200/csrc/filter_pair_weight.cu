@@ -232,7 +232,7 @@ cudaError_t launch_rows(bool fused, const PairMaps& m, const PairArgs& a, int z0
     using M = WeightSmem<ROWS, RAWP>;
     const size_t smem = M::bytes(a.syr);
     auto kern = fused ? nlm_pair_weight_kernel<ROWS, RAWP, true> : nlm_pair_weight_kernel<ROWS, RAWP, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory(kern, smem);
     if (e != cudaSuccess) return e;
     // a plane per grid z, of which a launch takes 65535
     for (int z = z0; z < z1; z += kPairGridZ) {

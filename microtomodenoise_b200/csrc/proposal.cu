@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "common.cuh"
 #include "proposal.cuh"
 
 namespace inlm {
@@ -849,8 +850,7 @@ cudaError_t net_backward(const NetLayout& L, const __nv_bfloat16* wb, const floa
     const int n_tiles = (int)nvox(lv[3]);
     const size_t hsm = (size_t)L.S * 4;
     if (hsm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(net_head_train_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
+        cudaError_t e = allow_shared_memory(net_head_train_kernel, hsm);
         if (e != cudaSuccess) return e;
     }
     net_head_train_kernel<<<n_tiles, 256, hsm, st>>>(act.a4, L.S, wb + L.wh, wf + L.bh, target, inv_n,
@@ -942,8 +942,7 @@ cudaError_t net_select(const NetLayout& L, const __nv_bfloat16* wb, const float*
     if (n_tiles <= 0) return cudaSuccess;
     const size_t sm = (size_t)kSelWarps * ((L.S + 3) / 4 * 4 + 256) * 4;
     if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(net_select_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_shared_memory(net_select_kernel, sm);
         if (e != cudaSuccess) return e;
     }
     const long long blocks = ((long long)n_tiles + kSelWarps - 1) / kSelWarps;
@@ -959,8 +958,7 @@ cudaError_t net_select_group(const NetLayout& L, const __nv_bfloat16* wb, const 
     const long long n_groups = (long long)gx * t8.y * t8.z;
     if (n_groups <= 0) return cudaSuccess;
     const size_t sm = (size_t)kSelWarps * (2 * ((L.S + 3) / 4 * 4) + 256) * 4;
-    cudaError_t e = cudaFuncSetAttribute(net_select_group_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_shared_memory(net_select_group_kernel, sm);
     if (e != cudaSuccess) return e;
     const long long blocks = (n_groups + kSelWarps - 1) / kSelWarps;
     net_select_group_kernel<<<(unsigned)blocks, 32 * kSelWarps, sm, st>>>(

@@ -278,8 +278,7 @@ static cudaError_t launch_tc(const float* in, Dim3i li, float* out, Dim3i lo, co
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = (int)std::min<long long>(tiles, sms);
-    cudaError_t e = cudaFuncSetAttribute(net_conv_tc_kernel<STRIDE, DGRAD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+    cudaError_t e = allow_shared_memory(net_conv_tc_kernel<STRIDE, DGRAD>, kTcSmem);
     if (e != cudaSuccess) return e;
     net_conv_tc_kernel<STRIDE, DGRAD><<<grid, kTcM, kTcSmem, st>>>(in, li, out, lo, W, b, act, err);
     return cudaGetLastError();

@@ -2,6 +2,7 @@
 used for both offsets of a pair. Bit-exact to the oracle at the edges of its
 tiles, z chunks, blocks and row forms, and where it has no workspace."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -193,6 +194,47 @@ def test_paired_handles_take_turns_on_one_workspace(gpu):
         g.free_device()
     _lib.check(L.inlm_debug_live_allocations(C.byref(live)), "live allocations")
     assert live.value == before
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form,sr", [(None, (4, 4, 4)), ("tile", (3, 4))])
+def test_threads_whose_launches_differ_in_shared_memory(gpu, form, sr):
+    """Launches of one kernel from several threads, with more and with less dynamic
+    shared memory: by the volume's depth (paired form) or the search radius."""
+    jobs = [((8 + 16 * i, 40, 64), (sr[i % len(sr)],) * 3) for i in range(4)]
+    handles, raws, got, errors = [], [], {}, []
+    for i, (shape, s) in enumerate(jobs):
+        g = IterativeNLM_GPU()
+        g.configure_device(shape, DenoiseParameters(radius_patchspace=(2, 2, 2), radius_searchspace=s))
+        if form:
+            g.select_tile_form(form)
+        g.set_sigma(_sigmas(shape[0])[1])
+        handles.append(g)
+        raws.append(synth.small_case(shape, seed=30 + i))
+    assert len({g.describe().split("smem=")[1].split()[0] for g in handles}) > 1
+    alone = []
+    for g, raw in zip(handles, raws):
+        g.Run_GaussianNoise(1, raw)
+        alone.append(g.get_result())
+
+    def work(i):
+        try:
+            for _ in range(60):
+                handles[i].Run_GaussianNoise(1, raws[i])
+            got[i] = handles[i].get_result()
+        except _lib.InlmError as e:
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for g in handles:
+        g.free_device()
+    assert not errors, errors
+    for i, want in enumerate(alone):
+        assert np.array_equal(got[i], want), jobs[i]
 
 
 @pytest.mark.gpu
