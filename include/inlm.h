@@ -181,11 +181,14 @@ int inlm_debug_wait_expiry(inlm_denoiser* d, int64_t cycles);
  * a workspace of `bytes` on a B200 (no device needed), whether the form runs, the
  * time of its plan and that of the whole volume in one chunk (the same unit), the
  * plan's bytes, its block's x and y, planes per chunk and per tile.
+ * inlm_debug_pair_pool bounds the workspaces that the process keeps on a device
+ * (0: an eighth of its memory).
  * inlm_debug_weight_mismatches compares, on the current
  * device, the form's weight step with the other kernels' for every float x in
  * [-3.6, -0] and stores how many differ. */
 int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes);
 int inlm_debug_weight_mismatches(int64_t* n);
+int inlm_debug_pair_pool(int64_t bytes);
 int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, int64_t bytes, double out[8]);
 
 /* Number of kernels this handle has launched since creation. */

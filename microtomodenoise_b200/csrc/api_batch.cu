@@ -268,7 +268,7 @@ struct inlm_batch {
     std::vector<float*> in;            // owned input volumes (the graph reads these)
     std::vector<float*> sigma_manual;  // manual mode: sigma[1] per slice
     std::vector<int> kind;             // batch body per volume (-1: own launch)
-    PairLoan pair;                     // workspace of the volumes in the paired form
+    PairBuf* pair = nullptr;           // workspace of the volumes in the paired form
     std::vector<int> order;            // batched volumes, heaviest tiles first
     // persistent launch groups: volumes of one patch shape whose shared
     // memory allows the same number of CTAs per SM
@@ -301,7 +301,7 @@ static void batch_free(inlm_batch* b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     for (inlm_denoiser* d : b->d)
         if (d) inlm_denoiser_destroy(d);
-    pair_give_back(&b->pair);
+    pair_give_back(b->pair);
     for (float* p : b->in) device_free(p);
     for (float* p : b->sigma_manual) device_free(p);
     device_free(b->d_counters);
@@ -478,11 +478,11 @@ extern "C" int inlm_batch_create(int n, const int* shapes, const inlm_params* pa
         if (d->pair.active && (long long)((d->shape[0] + 31) / 32) * ((d->shape[1] + 7) / 8) *
                                       ((d->shape[2] + 7) / 8) >= sms_dev) {
             const size_t bytes = d->pair.bytes;
-            if (bytes > b->pair.bytes) {
-                pair_give_back(&b->pair);
-                if (pair_take(dev, bytes, &b->pair) != INLM_OK) b->pair = PairLoan();
+            if (!b->pair || bytes > b->pair->bytes) {
+                pair_give_back(b->pair);
+                b->pair = pair_take(dev, bytes, true);
             }
-            if (b->pair.p) {
+            if (b->pair) {
                 paired.push_back(v);
                 continue;  // kind stays -1
             }
@@ -519,8 +519,8 @@ extern "C" int inlm_batch_create(int n, const int* shapes, const inlm_params* pa
         return bail(fail(INLM_ERR_CUDA, "batch setup failed"));
     // (volumes left without a workspace keep their single-pass launch)
     for (int v : paired) {
-        if (!b->pair.p || b->d[v]->pair.bytes > b->pair.bytes) continue;
-        const int rc = pair_share(b->d[v], b->pair.p);
+        if (!b->pair || b->d[v]->pair.bytes > b->pair->bytes) continue;
+        const int rc = pair_share(b->d[v], b->pair);
         if (rc) return bail(rc);
     }
 

@@ -11,6 +11,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -145,6 +146,20 @@ struct ProposalRun {
     inlm::DevBuf a1, a2, a3, a4, bitmap, pmass, counters, scale, plan_start, plan_off, mass_sum;
 };
 
+struct inlm_denoiser;
+
+// A workspace of the paired-offset FP32 form (api_pair.cu's pool).
+struct PairBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+    int users = 0;               // calls that hold it
+    bool alone = false;          // held by one owner that orders its passes itself
+    std::mutex enqueue;          // one pass at a time is enqueued
+    cudaEvent_t done = nullptr;  // end of the last pass enqueued
+    const inlm_denoiser* last = nullptr;  // whose pass that was
+};
+
 // Paired-offset FP32 form (api_pair.cu): its plan and workspace.
 struct PairRun {
     bool active = false;   // filters of this handle run the paired form
@@ -159,9 +174,8 @@ struct PairRun {
     size_t limit = 0;       // bound on the workspace set by a test (0: none)
     bool forced = false;    // the form runs within it whether or not that is faster
     size_t bytes = 0;       // workspace the plan needs
-    void* dist = nullptr;   // borrowed workspace (pair_idle hands it back)
-    size_t dist_bytes = 0;
-    bool shared = false;    // bound to a workspace somebody else holds (a batch)
+    PairBuf* dist = nullptr;  // borrowed workspace (pair_idle hands it back)
+    bool shared = false;    // it is somebody else's (a batch's)
     bool user = false;      // counted among the pool's users
 };
 
@@ -243,23 +257,20 @@ int encode_map_f32(CUtensorMap* tm, const void* base, int rank, const long long*
 // configuration) and plans its passes, borrows their workspace, runs one filter
 // pass, hands the workspace back (the handle's work on the GPU has ended),
 // releases everything (the form no longer runs).
-// pair_trim frees the workspace no handle has borrowed (true if there was one).
+// pair_trim frees the workspaces no handle has borrowed (true if there was one).
 int pair_configure(inlm_denoiser* d);
 int pair_prepare(inlm_denoiser* d, bool* ready);
 int pair_filter(inlm_denoiser* d);
 void pair_idle(inlm_denoiser* d);
 void pair_release(inlm_denoiser* d);
 bool pair_trim(int device);
-// One workspace for several handles whose passes run one after another (a
-// batch): a loan for the largest plan, the handles bound to it.
-struct PairLoan {
-    void* p = nullptr;
-    size_t bytes = 0;
-    int device = 0;
-};
-int pair_take(int device, size_t bytes, PairLoan* loan);
-void pair_give_back(PairLoan* loan);
-int pair_share(inlm_denoiser* d, void* ws);
+// One workspace for several handles: taken for the largest plan (null: no room),
+// handles bound to it (until they are gone, which is before it is given back).
+// alone: the owner's handles run on one stream (a captured batch), else their
+// passes are ordered by the workspace's event.
+PairBuf* pair_take(int device, size_t bytes, bool alone);
+void pair_give_back(PairBuf* b);
+int pair_share(inlm_denoiser* d, PairBuf* b);
 int pad_into(inlm_denoiser* d, const float* src, float* dst);
 int pad_into_half(inlm_denoiser* d, const float* src, void* dst);
 // Noise estimate of a device volume into d_dst (nz floats, device); host_copy

@@ -1,5 +1,7 @@
 // Host side of the paired-offset FP32 form (filter_pair.cu): when it applies,
 // the workspace and how a volume is cut into blocks and z chunks that fit it.
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -19,58 +21,107 @@ constexpr int kWorkspaceShare = 8;
 
 // Workspaces are not the handles': a call borrows one and hands it back when
 // its work on the GPU has ended, so handles that take turns share one buffer.
-// Per device the pool keeps at most one idle buffer, and none once the last
-// handle that borrowed is gone.
+// Per device the pool holds as many as calls in flight need, up to the share
+// above in total; from then on a call joins a buffer that is out, and the passes
+// on it run one after another (each fills the GPU). Nothing is allocated or freed
+// between the passes of such calls. None is left once the last handle that
+// borrowed is gone.
 struct Pool {
-    void* idle = nullptr;
-    size_t idle_bytes = 0;
+    std::vector<PairBuf*> bufs;
     int users = 0;
+    size_t share = 0;  // bytes kept in total
 };
 constexpr int kMaxDevices = 64;
 Pool g_pool[kMaxDevices];
 std::recursive_mutex g_pool_mutex;  // device_malloc may call pair_trim under it
+std::atomic<long long> g_pool_bound{0};  // a test's bound in place of the share
 
-cudaError_t borrow(int device, size_t bytes, void** p, size_t* got) {
-    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
-    Pool& pool = g_pool[device];
-    if (pool.idle && pool.idle_bytes < bytes) {
-        device_free(pool.idle);
-        pool.idle = nullptr;
-    }
-    if (pool.idle) {
-        *p = pool.idle;
-        *got = pool.idle_bytes;
-        pool.idle = nullptr;
-        return cudaSuccess;
-    }
-    const cudaError_t e = device_malloc(p, bytes);
-    if (e == cudaSuccess) *got = bytes;
-    return e;
+size_t pool_bytes(const Pool& pool) {
+    size_t n = 0;
+    for (const PairBuf* b : pool.bufs) n += b->bytes;
+    return n;
 }
 
-void hand_back(int device, void* p, size_t bytes) {
+size_t pool_share(const Pool& pool) {
+    const long long bound = g_pool_bound.load();
+    return bound > 0 ? (size_t)bound : pool.share;
+}
+
+// Frees the smallest idle buffer; false if there is none.
+bool free_idle(Pool& pool) {
+    PairBuf* least = nullptr;
+    for (PairBuf* b : pool.bufs)
+        if (b->users == 0 && (!least || b->bytes < least->bytes)) least = b;
+    if (!least) return false;
+    pool.bufs.erase(std::find(pool.bufs.begin(), pool.bufs.end(), least));
+    device_free(least->p);
+    cudaEventDestroy(least->done);
+    delete least;
+    return true;
+}
+
+PairBuf* borrow(int device, size_t bytes, bool alone) {
     std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
     Pool& pool = g_pool[device];
-    if (pool.users > 0 && (!pool.idle || pool.idle_bytes < bytes)) {
-        std::swap(p, pool.idle);
-        pool.idle_bytes = bytes;
+    if (pool.share == 0) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return nullptr;
+        pool.share = total_b / kWorkspaceShare;
     }
-    device_free(p);
+    PairBuf *idle = nullptr, *out = nullptr;
+    for (PairBuf* b : pool.bufs) {
+        if (b->bytes < bytes) continue;
+        if (b->users == 0 && (!idle || b->bytes < idle->bytes)) idle = b;
+        if (b->users > 0 && !b->alone && !alone && (!out || b->users < out->users)) out = b;
+    }
+    if (!idle) {
+        while (pool_bytes(pool) + bytes > pool_share(pool) && free_idle(pool)) {
+        }
+        if (pool_bytes(pool) + bytes <= pool_share(pool) || !out) {
+            PairBuf* b = new PairBuf();
+            b->device = device;
+            b->bytes = bytes;
+            if (device_malloc(&b->p, bytes) == cudaSuccess &&
+                cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) == cudaSuccess) {
+                pool.bufs.push_back(b);
+                idle = b;
+            } else {
+                cudaGetLastError();
+                device_free(b->p);
+                delete b;
+            }
+        }
+    }
+    PairBuf* b = idle ? idle : out;
+    if (!b) return nullptr;
+    b->alone = alone;
+    b->users++;
+    return b;
+}
+
+void hand_back(PairBuf* b) {
+    std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
+    Pool& pool = g_pool[b->device];
+    if (--b->users > 0) return;
+    b->last = nullptr;
+    while ((pool.users == 0 || pool_bytes(pool) > pool_share(pool)) && free_idle(pool)) {
+    }
 }
 
 void count_user(int device, int change) {
     std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
     Pool& pool = g_pool[device];
     pool.users += change;
-    if (pool.users == 0) {
-        device_free(pool.idle);
-        pool.idle = nullptr;
+    while (pool.users == 0 && free_idle(pool)) {
     }
 }
 
 size_t idle_bytes(int device) {
     std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
-    return g_pool[device].idle ? g_pool[device].idle_bytes : 0;
+    size_t n = 0;
+    for (const PairBuf* b : g_pool[device].bufs)
+        if (b->users == 0) n += b->bytes;
+    return n;
 }
 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
@@ -351,27 +402,21 @@ static int pair_bind(inlm_denoiser* d, void* ws) {
 static int pair_borrow(inlm_denoiser* d, bool* ok) {
     PairRun& r = d->pair;
     *ok = true;
-    if (r.dist || r.shared) return INLM_OK;
+    if (r.dist) return INLM_OK;
     if (!r.user) {
         count_user(d->device, 1);
         r.user = true;
     }
-    bool got = borrow(d->device, r.bytes, &r.dist, &r.dist_bytes) == cudaSuccess;
-    if (!got) {
-        cudaGetLastError();
+    r.dist = borrow(d->device, r.bytes, false);
+    if (!r.dist) {
         const size_t wanted = r.bytes;
         const int rc = pair_plan(d);
         if (rc) return rc;
-        got = r.active && r.bytes < wanted && borrow(d->device, r.bytes, &r.dist, &r.dist_bytes) == cudaSuccess;
+        if (r.active && r.bytes < wanted) r.dist = borrow(d->device, r.bytes, false);
         r.active = true;  // a later call may find room again
     }
-    if (!got) {
-        cudaGetLastError();
-        r.dist = nullptr;
-        *ok = false;
-        return INLM_OK;
-    }
-    return pair_bind(d, r.dist);
+    *ok = r.dist != nullptr;
+    return r.dist ? pair_bind(d, r.dist->p) : INLM_OK;
 }
 
 // Borrows the workspace of the handle's passes; *ready = false when the form does
@@ -381,8 +426,7 @@ int inlm::pair_prepare(inlm_denoiser* d, bool* ready) {
     return d->pair.active ? pair_borrow(d, ready) : INLM_OK;
 }
 
-// Enqueues one filter pass.
-int inlm::pair_filter(inlm_denoiser* d) {
+static int pair_launches(inlm_denoiser* d) {
     const PairRun& r = d->pair;
     const int* pr = d->geo.patch_radius;
     const bool fused = d->p.precision == INLM_PRECISION_F32_FMA;
@@ -411,42 +455,52 @@ int inlm::pair_filter(inlm_denoiser* d) {
     return INLM_OK;
 }
 
-int inlm::pair_share(inlm_denoiser* d, void* ws) {
+// Enqueues one filter pass, after the last pass of another handle on the same
+// workspace.
+int inlm::pair_filter(inlm_denoiser* d) {
+    PairBuf* b = d->pair.dist;
+    if (b->alone) return pair_launches(d);
+    std::lock_guard<std::mutex> lock(b->enqueue);
+    if (b->last && b->last != d) CUDA_TRY(cudaStreamWaitEvent(d->stream, b->done, 0));
+    const int rc = pair_launches(d);
+    b->last = d;  // (whatever was enqueued counts)
+    CUDA_TRY(cudaEventRecord(b->done, d->stream));
+    return rc;
+}
+
+int inlm::pair_share(inlm_denoiser* d, PairBuf* b) {
     pair_idle(d);
     d->pair.shared = true;
-    return pair_bind(d, ws);
+    d->pair.dist = b;
+    return pair_bind(d, b->p);
 }
 
-int inlm::pair_take(int device, size_t bytes, PairLoan* loan) {
+PairBuf* inlm::pair_take(int device, size_t bytes, bool alone) {
     count_user(device, 1);
-    if (borrow(device, bytes, &loan->p, &loan->bytes) == cudaSuccess) {
-        loan->device = device;
-        return INLM_OK;
-    }
-    cudaGetLastError();
-    loan->p = nullptr;
-    count_user(device, -1);
-    return INLM_ERR_NOMEM;
+    PairBuf* b = borrow(device, bytes, alone);
+    if (!b) count_user(device, -1);
+    return b;
 }
 
-void inlm::pair_give_back(PairLoan* loan) {
-    if (!loan->p) return;
-    hand_back(loan->device, loan->p, loan->bytes);
-    count_user(loan->device, -1);
-    loan->p = nullptr;
+void inlm::pair_give_back(PairBuf* b) {
+    if (!b) return;
+    const int device = b->device;
+    hand_back(b);
+    count_user(device, -1);
 }
 
 bool inlm::pair_trim(int device) {
     std::lock_guard<std::recursive_mutex> lock(g_pool_mutex);
-    if (device < 0 || device >= kMaxDevices || !g_pool[device].idle) return false;
-    device_free(g_pool[device].idle);
-    g_pool[device].idle = nullptr;
-    return true;
+    if (device < 0 || device >= kMaxDevices) return false;
+    bool any = false;
+    while (free_idle(g_pool[device])) any = true;
+    return any;
 }
 
 void inlm::pair_idle(inlm_denoiser* d) {
     PairRun& r = d->pair;
-    if (r.dist) hand_back(d->device, r.dist, r.dist_bytes);
+    if (!r.dist || r.shared) return;
+    hand_back(r.dist);
     r.dist = nullptr;
 }
 
@@ -469,6 +523,12 @@ extern "C" int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes) {
     d->pair.limit = (size_t)std::llabs(bytes);
     d->pair.forced = bytes > 0;
     return pair_plan(d);
+}
+
+extern "C" int inlm_debug_pair_pool(int64_t bytes) {
+    if (bytes < 0) return fail(INLM_ERR_ARG, "bad argument");
+    g_pool_bound.store(bytes);
+    return INLM_OK;
 }
 
 extern "C" int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, int64_t bytes, double out[8]) {

@@ -238,6 +238,54 @@ def test_threads_whose_launches_differ_in_shared_memory(gpu, form, sr):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bound", [1, 0])
+def test_threads_share_workspaces(gpu, bound):
+    """Jobs of several threads at a time: with one workspace between them (they join
+    the one that is out, pass after pass) and with one each; the pool keeps none
+    beyond its bound, and none when the last handle is gone."""
+    L = _lib.load()
+
+    def live():
+        n = C.c_int64(0)
+        _lib.check(L.inlm_debug_live_allocations(C.byref(n)), "live allocations")
+        return n.value
+
+    before = live()
+    cases = [((24, 40, 64), (2, 2, 2), (4, 4, 4)), ((24, 40, 64), (2, 2, 2), (4, 4, 4)),
+             ((30, 33, 70), (1, 1, 1), (4, 4, 4)), ((16, 48, 48), (3, 3, 3), (3, 3, 3))]
+    handles, raws, alone, got = [], [], [], {}
+    for i, (shape, pr, sr) in enumerate(cases):
+        g = IterativeNLM_GPU()
+        g.configure_device(shape, DenoiseParameters(radius_patchspace=pr, radius_searchspace=sr, noise_mode="manual",
+                                                    sigma=(0.06, 0.05), maxiterations=4))
+        handles.append(g)
+        raws.append(synth.small_case(shape, seed=20 + i))
+        g.denoise(raws[i])  # (a handle's later jobs start from sigma[1])
+        alone.append(g.denoise(raws[i])[0])
+        assert "paired" in g.describe()
+    held = live()
+
+    def work(i):
+        got[i] = [handles[i].denoise(raws[i])[0] for _ in range(12)]
+
+    _lib.check(L.inlm_debug_pair_pool(bound), "pair_pool")
+    try:
+        ts = [threading.Thread(target=work, args=(i,)) for i in range(len(cases))]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        assert live() <= (held if bound else held + len(cases))
+        for i, want in enumerate(alone):
+            assert len(got[i]) == 12 and all(np.array_equal(o, want) for o in got[i]), cases[i]
+    finally:
+        L.inlm_debug_pair_pool(0)
+    for g in handles:
+        g.free_device()
+    assert live() == before
+
+
+@pytest.mark.gpu
 def test_weight_step_equals_the_other_kernels_for_every_argument(gpu):
     n = C.c_int64(-1)
     _lib.check(_lib.load().inlm_debug_weight_mismatches(C.byref(n)), "weight_mismatches")
