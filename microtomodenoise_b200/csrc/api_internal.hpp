@@ -254,11 +254,12 @@ int upload_sigma_device(inlm_denoiser* d);
 int encode_map_f32(CUtensorMap* tm, const void* base, int rank, const long long* dims, const long long* pitch,
                    const int* box);
 // Paired-offset form: decides whether it covers the handle (after the tile
-// configuration) and plans its passes, borrows their workspace, runs one filter
+// configuration), plans its passes for the memory there is, borrows their workspace, runs one filter
 // pass, hands the workspace back (the handle's work on the GPU has ended),
 // releases everything (the form no longer runs).
 // pair_trim frees the workspaces no handle has borrowed (true if there was one).
 int pair_configure(inlm_denoiser* d);
+int pair_plan(inlm_denoiser* d);
 int pair_prepare(inlm_denoiser* d, bool* ready);
 int pair_filter(inlm_denoiser* d);
 void pair_idle(inlm_denoiser* d);

@@ -277,7 +277,7 @@ bool pair_extents(const Geometry& g, const int shape[3], int nslices, size_t sme
 
 // Plans the handle's passes for the memory there is; the handle runs the form where
 // the plan is faster than the single-pass kernel.
-static int pair_plan(inlm_denoiser* d) {
+int inlm::pair_plan(inlm_denoiser* d) {
     PairRun& r = d->pair;
     PairArgs& a = r.args;
     const int* pr = d->geo.patch_radius;

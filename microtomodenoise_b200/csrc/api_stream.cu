@@ -48,6 +48,7 @@ struct StreamJob {
     float rel_mass = 0.f;  // relative fallback (the mean over each sub-volume's lists)
     std::vector<int> sched_k;  // per-iteration schedule (inlm_proposal_schedule), or empty
     std::vector<float> sched_rel;
+    PairBuf* pair = nullptr;  // workspace of the denoisers in the paired form
 
     ~StreamJob() {
         for (auto& kv : pairs)
@@ -55,6 +56,7 @@ struct StreamJob {
                 if (kv.second.d[j]) inlm_denoiser_destroy(kv.second.d[j]);
                 device_free(kv.second.stage[j]);
             }
+        pair_give_back(pair);
         if (noise) inlm_noise_destroy(noise);
         device_free(d_sig0);
         device_free(d_sig);
@@ -100,6 +102,30 @@ int get_pair(StreamJob& J, const inlm_params& p, int depth, inlm_proposal* net, 
         }
     }
     *out = &sp;
+    return INLM_OK;
+}
+
+// One workspace for all denoisers of a job, taken when all of them exist: planned
+// for the memory that is left, and neither allocated nor freed between slabs. Their
+// passes follow one another (each fills the GPU); copies overlap as before. Where
+// there is no room for it, each pass looks for its own.
+int take_workspace(StreamJob& J, int device) {
+    size_t most = 0;
+    for (auto& kv : J.pairs)
+        for (inlm_denoiser* d : kv.second.d) {
+            if (!d->pair.active) continue;
+            const int rc = pair_plan(d);
+            if (rc) return rc;
+            if (d->pair.active) most = std::max(most, d->pair.bytes);
+        }
+    if (most > 0) J.pair = pair_take(device, most, false);
+    if (!J.pair) return INLM_OK;
+    for (auto& kv : J.pairs)
+        for (inlm_denoiser* d : kv.second.d) {
+            if (!d->pair.active) continue;
+            const int rc = pair_share(d, J.pair);
+            if (rc) return rc;
+        }
     return INLM_OK;
 }
 
@@ -266,6 +292,12 @@ extern "C" int inlm_stream_denoise_sched(const int shape[3], const inlm_params* 
 
     CUDA_TRY(dalloc(&J.d_sig0, nz));
     CUDA_TRY(dalloc(&J.d_sig, nz));
+    for (int z0 : z0s) {
+        SlabPair* sp;
+        int rc = get_pair(J, *p, std::min(nz, std::min(nz, z0 + sd) + halo) - std::max(0, z0 - halo), net, k, min_mass,
+                          &sp);
+        if (rc) return rc;
+    }
     int nwin = 0;
     if (!manual) {
         int rc = inlm_noise_create(shape, p->n_samples, p->noise_patchsize, p->noise_seed,
@@ -277,6 +309,8 @@ extern "C" int inlm_stream_denoise_sched(const int shape[3], const inlm_params* 
         rc = noise_prepare(J.noise, p, &nwin, nullptr);
         if (rc) return rc;
     }
+    int wrc = take_workspace(J, p->device_id);
+    if (wrc) return wrc;
     double h2d = 0, d2h = 0;
     cudaEvent_t t0, t1;
     CUDA_TRY(cudaEventCreate(&t0));

@@ -3,10 +3,12 @@ in-memory schedule (inlm_denoise) bit for bit, whatever the slab depth,
 because each slab is filtered as a sub-volume whose halo covers every value
 its voxels read (and, for the FP16 and learned forms, whose tiles sit where
 the whole volume's do)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from microtomodenoise_b200 import DenoiseParameters, IterativeNLM_GPU, stream_denoise, synth
+from microtomodenoise_b200 import DenoiseParameters, IterativeNLM_GPU, _lib, stream_denoise, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -37,6 +39,41 @@ def test_stream_equals_in_memory(gpu, mode, slab, prec):
     if mode != "manual":
         assert np.array_equal(s0, w0) and np.array_equal(s1, w1)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("mode", ["manual", "global"])
+def test_stream_with_a_failing_allocation(gpu, mode):
+    """Each allocation of a streamed job fails once: the job ends with
+    INLM_ERR_NOMEM or, where it was the workspace shared by its slabs, without it,
+    with the same result; slab denoisers are all made before the first filter pass."""
+    L = _lib.load()
+
+    def live():
+        n = C.c_int64(0)
+        _lib.check(L.inlm_debug_live_allocations(C.byref(n)), "live allocations")
+        return n.value
+
+    raw = synth.small_case((44, 40, 56), seed=22)
+    p = DenoiseParameters(radius_patchspace=(2, 2, 2), radius_searchspace=(3, 3, 3), noise_mode=mode,
+                          sigma=(0.06, 0.05), noise_seed=3, n_samples=3000, maxiterations=2)
+    want = stream_denoise(raw, p, slab_depth=8)[0]
+    before, failed, passed = live(), 0, 0
+    for k in range(400):
+        L.inlm_debug_fail_allocation(k)
+        try:
+            got = stream_denoise(raw, p, slab_depth=8)[0]
+        except _lib.InlmError as e:
+            assert e.code == -4, e
+            failed += 1
+        else:
+            assert np.array_equal(got, want), k
+            passed += 1
+        finally:
+            L.inlm_debug_fail_allocation(-1)
+        assert live() == before, k
+        if passed > 4:  # past the last allocation
+            break
+    assert failed > 10 and passed > 4
 
 
 def test_stream_continuous_estimate(gpu):
