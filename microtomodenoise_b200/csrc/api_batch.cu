@@ -442,7 +442,6 @@ extern "C" int inlm_batch_create(int n, const int* shapes, const inlm_params* pa
     b->in.assign(n, nullptr);
     b->sigma_manual.assign(n, nullptr);
     b->kind.assign(n, -1);
-    std::vector<int> paired;  // volumes that run the paired form
     int sms_dev = 148;
     cudaDeviceGetAttribute(&sms_dev, cudaDevAttrMultiProcessorCount, dev);
     for (int v = 0; v < n; v++) {
@@ -471,22 +470,35 @@ extern "C" int inlm_batch_create(int n, const int* shapes, const inlm_params* pa
             rc = estimate_into(d, b->in[v], d->d_sigma0, nullptr);
             if (rc) return bail(rc);
         }
-        // A volume of at least one tile per SM runs the paired form in its own
-        // launches, one volume after another on the main stream: measured 1.4
-        // times the persistent bodies and single-pass launches on six volumes of
-        // 29 thousand to 1.9 million voxels. Its workspace is taken below.
-        if (d->pair.active && (long long)((d->shape[0] + 31) / 32) * ((d->shape[1] + 7) / 8) *
-                                      ((d->shape[2] + 7) / 8) >= sms_dev) {
-            const size_t bytes = d->pair.bytes;
-            if (!b->pair || bytes > b->pair->bytes) {
-                pair_give_back(b->pair);
-                b->pair = pair_take(dev, bytes, true);
-            }
-            if (b->pair) {
-                paired.push_back(v);
-                continue;  // kind stays -1
-            }
-        }
+    }
+    // A volume of at least one tile per SM runs the paired form in its own
+    // launches, one volume after another on the main stream: measured 1.4
+    // times the persistent bodies and single-pass launches on six volumes of
+    // 29 thousand to 1.9 million voxels. All share one workspace, the largest that
+    // there is room for now that every volume has its buffers; a volume that
+    // needs more than it is batched as if the form did not cover it.
+    std::vector<int> paired;
+    for (int v = 0; v < n; v++) {
+        inlm_denoiser* d = b->d[v];
+        if (!d->pair.active || (long long)((d->shape[0] + 31) / 32) * ((d->shape[1] + 7) / 8) *
+                                       ((d->shape[2] + 7) / 8) < sms_dev)
+            continue;
+        const int rc = pair_plan(d);
+        if (rc) return bail(rc);
+        if (d->pair.active) paired.push_back(v);
+    }
+    std::stable_sort(paired.begin(), paired.end(),
+                     [&](int x, int y) { return b->d[x]->pair.bytes > b->d[y]->pair.bytes; });
+    for (int v : paired) {
+        if (!b->pair) b->pair = pair_take(dev, b->d[v]->pair.bytes, true);
+        if (!b->pair) continue;
+        const int rc = pair_share(b->d[v], b->pair);
+        if (rc) return bail(rc);
+    }
+    for (int v = 0; v < n; v++) {
+        inlm_denoiser* d = b->d[v];
+        int rc = INLM_OK;
+        if (d->pair.shared) continue;  // kind stays -1
         // A volume whose own configuration is the column form, the 16-deep
         // CTA or the warp-specialised kernel (faster than the persistent
         // depth-8 body) and which fills the GPU by itself (>= 4 waves of CTAs)
@@ -517,12 +529,6 @@ extern "C" int inlm_batch_create(int n, const int* shapes, const inlm_params* pa
     }
     if (cudaStreamSynchronize(b->stream) != cudaSuccess)
         return bail(fail(INLM_ERR_CUDA, "batch setup failed"));
-    // (volumes left without a workspace keep their single-pass launch)
-    for (int v : paired) {
-        if (!b->pair || b->d[v]->pair.bytes > b->pair->bytes) continue;
-        const int rc = pair_share(b->d[v], b->pair);
-        if (rc) return bail(rc);
-    }
 
     // batched volumes, heaviest tile first (longest-processing-time order)
     int nb = 0;

@@ -3,10 +3,12 @@ whole schedule captured as a CUDA graph) and the tile-configuration
 autotuner. Every batched volume must equal its own single-volume run of the
 same schedule bit for bit: the persistent kernel runs the same tile bodies,
 and the noise estimates draw the same samples."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from microtomodenoise_b200 import Batch, DenoiseParameters, IterativeNLM_GPU, synth
+from microtomodenoise_b200 import Batch, DenoiseParameters, IterativeNLM_GPU, _lib, synth
 from oracle.oracle import FilterParams
 
 pytestmark = pytest.mark.gpu
@@ -165,3 +167,43 @@ def test_batch_at_config3_sizes_against_the_oracle(gpu, port):
         assert np.array_equal(o1.ravel()[vox], want1), f"iteration 1, shape {raw.shape}"
         want2 = port.filter_voxels(raw_pad, port.pad_reflective(o1, pad), raw.shape, p, s1, vox)
         assert np.array_equal(o2.ravel()[vox], want2), f"iteration 2, shape {raw.shape}"
+
+
+def test_paired_volumes_share_one_workspace_and_may_lose_it(gpu):
+    """Volumes of a tile per SM or more run the paired form on one workspace. Each
+    allocation of the batch's creation fails once: creation ends with
+    INLM_ERR_NOMEM, or the workspace was the one that failed and the volumes run on
+    a smaller one, or on none, with the same results."""
+    L = _lib.load()
+
+    def live():
+        n = C.c_int64(0)
+        _lib.check(L.inlm_debug_live_allocations(C.byref(n)), "live allocations")
+        return n.value
+
+    cs = [(s, DenoiseParameters(radius_patchspace=(pr,) * 3, radius_searchspace=(sr,) * 3, noise_mode="manual",
+                                sigma=(0.05, 0.04), maxiterations=2))
+          for s, pr, sr in [((32, 64, 160), 1, 3), ((40, 72, 160), 2, 3), ((12, 30, 40), 2, 2), ((34, 64, 200), 1, 5)]]
+    raws = [synth.small_case(s, seed=40 + i) for i, (s, _) in enumerate(cs)]
+    want = [single(raw, p) for raw, (_, p) in zip(raws, cs)]
+    before, seen, done = live(), set(), 0
+    for k in range(400):
+        L.inlm_debug_fail_allocation(k)
+        try:
+            b = Batch([s for s, _ in cs], [p for _, p in cs])
+        except _lib.InlmError as e:
+            assert e.code == -4, e
+            assert live() == before, k
+            continue
+        finally:
+            L.inlm_debug_fail_allocation(-1)
+        n = b.describe().count("own launch paired")
+        seen.add(n)
+        for got, w in zip(b.run(raws), want):
+            assert np.array_equal(got, w), (k, b.describe())
+        b.close()
+        assert live() == before, k
+        done += n == 3
+        if done == 3:  # past the last allocation
+            break
+    assert seen >= {2, 3} and done == 3, seen
