@@ -1477,7 +1477,7 @@ extern "C" int inlm_describe(inlm_denoiser* d, char* buf, size_t len) {
                  g.pad[1], g.pad[2]);
     }
     else if (d->pair.active)
-        snprintf(buf, len, "nlm_tile_f32%s_paired<%d,%d,%d> tz=%d raw_global smem=%zu S=%zu P=%zu weights=%s pad=%d,%d,%d",
+        snprintf(buf, len, "nlm_tile_f32%s_paired<%d,%d,%d> tz=%d raw_planes smem=%zu S=%zu P=%zu weights=%s pad=%d,%d,%d",
                  d->p.precision == INLM_PRECISION_F32_FMA ? "_fused" : "", g.patch_radius[0], g.patch_radius[1],
                  g.patch_radius[2], d->pair.args.tz, pair_smem_bytes(g.patch_radius[0], g.patch_radius[2], d->pair.args), g.search.size(), g.taps.size(),
                  g.specialised && d->p.weight_table == INLM_WEIGHTS_CPU ? "cpu-table" : "distweight",
