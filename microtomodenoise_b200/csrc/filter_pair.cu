@@ -262,7 +262,10 @@ __global__ void __launch_bounds__(32 * PairSmem<RX, RZ>::kWarps, 1)
     }
     const bool arrived = mbar_wait_bounded(bar, 0);
     if (!__syncthreads_and(arrived)) {
-        if (tid == 0) set_error(a.err, DEV_TMA_TIMEOUT);
+        if (tid == 0) {
+            set_error(a.err, DEV_TMA_TIMEOUT);
+            mbar_wait_bounded(bar, 0);  // let the copy land before the CTA's memory goes away
+        }
         return;
     }
     const int pplane = PBX * a.pby;
