@@ -185,9 +185,12 @@ int inlm_debug_wait_expiry(inlm_denoiser* d, int64_t cycles);
  * (0: an eighth of its memory).
  * inlm_debug_weight_mismatches compares, on the current
  * device, the form's weight step with the other kernels' for every float x in
- * [-3.6, -0] and stores how many differ. */
+ * [-3.6, -0] and stores how many differ; inlm_debug_fused_weight_error stores the
+ * largest relative error of the fused form's step over the x that it weighs,
+ * against 64 bits. */
 int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes);
 int inlm_debug_weight_mismatches(int64_t* n);
+int inlm_debug_fused_weight_error(double* worst);
 int inlm_debug_pair_pool(int64_t bytes);
 int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, int64_t bytes, double out[8]);
 

@@ -548,16 +548,29 @@ extern "C" int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, in
     return INLM_OK;
 }
 
+// Runs a check that leaves one 64-bit value on the device (from zero).
+template <class T, class F>
+static int device_check(T* out, F launch) {
+    static_assert(sizeof(T) == 8, "one 64-bit value");
+    T* p = nullptr;
+    CUDA_TRY(dalloc(&p, 1));
+    cudaError_t e = cudaMemset(p, 0, sizeof(T));
+    if (e == cudaSuccess) e = launch(p);
+    if (e == cudaSuccess) e = cudaMemcpy(out, p, sizeof(T), cudaMemcpyDeviceToHost);
+    device_free(p);
+    CUDA_TRY(e);
+    return INLM_OK;
+}
+
 extern "C" int inlm_debug_weight_mismatches(int64_t* n) {
     if (!n) return fail(INLM_ERR_ARG, "null argument");
-    unsigned long long* dn = nullptr;
-    CUDA_TRY(dalloc(&dn, 1));
     unsigned long long h = 0;
-    cudaError_t e = cudaMemset(dn, 0, sizeof h);
-    if (e == cudaSuccess) e = launch_weight_mismatches(dn, -0.0f, nullptr);
-    if (e == cudaSuccess) e = cudaMemcpy(&h, dn, sizeof h, cudaMemcpyDeviceToHost);
-    device_free(dn);
-    CUDA_TRY(e);
-    *n = (int64_t)h;
-    return INLM_OK;
+    const int rc = device_check(&h, [](unsigned long long* p) { return launch_weight_mismatches(p, -0.0f, nullptr); });
+    if (rc == INLM_OK) *n = (int64_t)h;
+    return rc;
+}
+
+extern "C" int inlm_debug_fused_weight_error(double* worst) {
+    if (!worst) return fail(INLM_ERR_ARG, "null argument");
+    return device_check(worst, [](double* p) { return launch_fused_weight_error(p, nullptr); });
 }

@@ -73,5 +73,8 @@ cudaError_t launch_pair_weights(bool fused, const PairMaps& m, const PairArgs& a
 // Counts the x in [-3.6, -0] whose exact_weight_pair_fast step differs from
 // exact_weight_pair's.
 cudaError_t launch_weight_mismatches(unsigned long long* n, float neg0, cudaStream_t st);
+// Raises *worst to the largest relative error of fused_weight_pair over the x that
+// it weighs (1e300: an x past the cutoff weighs something).
+cudaError_t launch_fused_weight_error(double* worst, cudaStream_t st);
 
 }  // namespace inlm

@@ -257,7 +257,39 @@ __global__ void __launch_bounds__(256) weight_mismatch_kernel(unsigned long long
     }
 }
 
+// Largest relative error of fused_weight_pair's weight over the x in
+// [-3.56648, -0], against the quotient in 64 bits (bits of a positive double); x
+// past the cutoff, -inf and NaN must weigh 0.
+__global__ void __launch_bounds__(256) fused_weight_error_kernel(unsigned long long* worst) {
+    const unsigned last = __float_as_uint(-3.56648f);
+    const f32x2 one = splat2(1.f);
+    auto weight = [&](float x) {
+        f32x2 acc = 0ull, sum = 0ull;
+        float max0 = 0.f, max1 = 0.f;
+        fused_weight_pair(splat2(x), one, make_float2(1.f, 1.f), acc, sum, max0, max1);
+        const float2 a = unpack2(acc), s = unpack2(sum);
+        return a.x == s.x && a.y == s.x && s.y == s.x && max0 == s.x && max1 == s.x ? s.x : __int_as_float(0x7fffffff);
+    };
+    double e = 0.0;
+    for (unsigned b = 0x80000000u + blockIdx.x * 256u + threadIdx.x; b < last; b += gridDim.x * 256u) {
+        const double x = (double)__uint_as_float(b);
+        const double q = (120.0 + x * (60.0 + x * (12.0 + x))) / (120.0 - x * (60.0 - x * (12.0 - x)));
+        const double d = fabs((double)weight(__uint_as_float(b)) - q) / q;
+        if (!(d <= e)) e = d == d ? d : 1e300;
+    }
+    if (threadIdx.x < 4) {
+        const float out[4] = {-3.56648f, -1e30f, -INFINITY, NAN};
+        if (!(weight(out[threadIdx.x]) == 0.f)) e = 1e300;
+    }
+    if (e > 0.0) atomicMax(worst, (unsigned long long)__double_as_longlong(e));
+}
+
 }  // namespace
+
+cudaError_t launch_fused_weight_error(double* worst, cudaStream_t st) {
+    fused_weight_error_kernel<<<148 * 8, 256, 0, st>>>(reinterpret_cast<unsigned long long*>(worst));
+    return cudaGetLastError();
+}
 
 cudaError_t launch_weight_mismatches(unsigned long long* n, float neg0, cudaStream_t st) {
     weight_mismatch_kernel<<<148 * 8, 256, 0, st>>>(n, neg0);

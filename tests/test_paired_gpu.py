@@ -292,6 +292,17 @@ def test_weight_step_equals_the_other_kernels_for_every_argument(gpu):
     assert n.value == 0
 
 
+@pytest.mark.gpu
+def test_fused_weight_step_for_every_argument(gpu):
+    """Bound: with u = 2^-24, 12 + x is off by 4.8e-7, the next two Horner steps by
+    3.57 times that of the one before and half an ulp of their own: 1.0e-5 on a
+    numerator of 13.3 at the cutoff (7.5e-7), 5.0e-5 on a denominator of 532 (0.9e-7);
+    the approximate reciprocal adds one ulp (1.2e-7) and the product u: 1.03e-6."""
+    worst = C.c_double(-1)
+    _lib.check(_lib.load().inlm_debug_fused_weight_error(C.byref(worst)), "fused_weight_error")
+    assert 0 < worst.value <= 1.1e-6
+
+
 @pytest.mark.parametrize("pr", [(1, 1, 1), (1, 1, 2), (2, 2, 1), (2, 2, 2), (3, 3, 2), (3, 3, 3)])
 @pytest.mark.parametrize("sr,nslices", [((3, 4, 2), 11), ((5, 5, 5), 7), ((10, 10, 10), 11), ((2, 7, 9), 15)])
 def test_offsets_come_in_mirrored_pairs(lib, pr, sr, nslices):
