@@ -489,6 +489,12 @@ int inlm_device_count(int* n);
 /* Free and total memory of a device in bytes (cudaMemGetInfo; the reference
  * sizes its blocks from it, iternlm_gpu.cu:1537-1566). */
 int inlm_device_memory(int device, size_t* free_bytes, size_t* total_bytes);
+/* The paired FP32 form keeps the workspaces of its last calls on a device, in all
+ * up to an eighth of its memory, while a denoiser that used one exists. The
+ * library's own allocations take them back when memory runs out; this call gives
+ * those that no call is using to the rest of the program. Later calls allocate
+ * anew. */
+int inlm_trim_memory(int device);
 
 /* ---------------- one iteration at a time over host-resident volumes ----------------
  * replaces the host-RAM overload of IterativeNLM_GPU::Run_GaussianNoise_GPUBlocks

@@ -26,7 +26,7 @@ from . import _lib
 from ._lib import InlmError, InlmParams, NOISE_MODES, PRECISIONS
 
 __all__ = ["DenoiseParameters", "IterativeNLM_GPU", "NoiseLevel", "Batch", "denoise",
-           "denoise_multi", "denoise_f64_blocks", "stream_denoise", "Blocks", "InlmError"]
+           "denoise_multi", "denoise_f64_blocks", "stream_denoise", "Blocks", "trim_memory", "InlmError"]
 
 
 @dataclass
@@ -494,6 +494,13 @@ class Blocks:
             self.close()
         except Exception:
             pass
+
+
+def trim_memory(device: int = 0) -> None:
+    """Gives the device memory that the paired FP32 form keeps between calls (up
+    to an eighth of the device's, while a denoiser that used it exists) back to the
+    rest of the program, torch for instance."""
+    _lib.check(_lib.load().inlm_trim_memory(device), "trim_memory")
 
 
 def denoise_multi(raw: np.ndarray, params: DenoiseParameters, device_ids, out: Optional[np.ndarray] = None):

@@ -49,7 +49,7 @@ EXPORTS = (
     "inlm_blocks_run_iteration", "inlm_blocks_attach_proposal", "inlm_stream_denoise_ex",
     "inlm_proposal_schedule", "inlm_stream_denoise_sched", "inlm_blocks_proposal_schedule", "inlm_device_memory", "inlm_debug_fail_allocation",
     "inlm_debug_live_allocations", "inlm_debug_wait_expiry", "inlm_debug_pair_workspace", "inlm_debug_weight_mismatches",
-    "inlm_debug_pair_plan", "inlm_debug_pair_pool", "inlm_debug_fused_weight_error",
+    "inlm_debug_pair_plan", "inlm_debug_pair_pool", "inlm_trim_memory", "inlm_debug_fused_weight_error",
     "inlm_denoise_f64_blocks",
 )
 
@@ -173,6 +173,7 @@ def load(path: str = "") -> C.CDLL:
     L.inlm_debug_pair_workspace.argtypes = [vp, C.c_int64]
     L.inlm_debug_weight_mismatches.argtypes = [C.POINTER(C.c_int64)]
     L.inlm_debug_fused_weight_error.argtypes = [C.POINTER(C.c_double)]
+    L.inlm_trim_memory.argtypes = [C.c_int]
     L.inlm_debug_pair_pool.argtypes = [C.c_int64]
     L.inlm_debug_pair_plan.argtypes = [C.c_int * 3, C.POINTER(InlmParams), C.c_int64, C.c_double * 8]
     L.inlm_denoise_f64_blocks.argtypes = [C.c_int * 3, C.POINTER(InlmParams), vp, C.c_int, vp, C.c_int, vp,

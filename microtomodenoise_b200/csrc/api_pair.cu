@@ -514,6 +514,12 @@ void inlm::pair_release(inlm_denoiser* d) {
     r.active = false;
 }
 
+extern "C" int inlm_trim_memory(int device) {
+    if (device < 0) return fail(INLM_ERR_ARG, "device %d", device);
+    pair_trim(device);
+    return INLM_OK;
+}
+
 extern "C" int inlm_debug_pair_workspace(inlm_denoiser* d, int64_t bytes) {
     if (!d) return fail(INLM_ERR_ARG, "null handle");
     if (!d->pair.offsets.p) return fail(INLM_ERR_UNSUPPORTED, "the paired form does not cover this handle");
