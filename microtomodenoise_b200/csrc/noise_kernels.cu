@@ -276,6 +276,7 @@ __device__ __forceinline__ void em_window(const float* __restrict__ values, int 
 constexpr int kEmClusterThreads = 512;
 constexpr int kEmManyThreads = 256, kEmManyValues = 40;  // the shape for many windows
 constexpr int kEmMaxCluster = 8;
+constexpr int kEmSms = 148;
 constexpr int kEmMaxValues = 28;  // per thread (64 registers at two CTAs per SM)
 
 struct __align__(16) EmPartial {
@@ -775,17 +776,21 @@ cudaError_t launch_noise_em(const float* values, const int2* windows, int n_wind
     // idle SMs: a pass is then shorter
     if (max_window > 0 && max_window <= (long long)kEmMaxCluster * kEmClusterThreads * kEmMaxValues) {
         int ctas = 1;
-        // many windows: half the threads with more samples each, so that the
-        // reductions take fewer of the issue slots (256 windows of up to 39000
-        // samples: 727 us against 794 us)
+        // Many windows: half the threads with more samples each, so that the
+        // reductions take fewer of the issue slots. It pays where the CTAs are at
+        // least 0.7 full and make two waves (three per SM); against 512 threads,
+        // us, by windows x samples: 256 x 39000 650 / 651, 256 x 31000 694 / 743,
+        // 600 x 32000 1241 / 1388, 600 x 80000 3516 / 3844, 1000 x 18000 1042 /
+        // 1133; below that 256 x 27000 631 / 491, 600 x 43000 2884 / 1959, and with
+        // fewer CTAs 300 x 18000 464 / 439, 600 x 9000 366 / 338.
         while ((long long)ctas * kEmManyThreads * kEmManyValues < max_window) ctas *= 2;
-        if (ctas <= kEmMaxCluster && (long long)n_windows * ctas >= 4 * 148 &&
-            max_window > (long long)ctas * kEmManyThreads * kEmManyValues / 2)
+        if (ctas <= kEmMaxCluster && (long long)n_windows * ctas >= 6 * kEmSms &&
+            10 * max_window >= 7ll * ctas * kEmManyThreads * kEmManyValues)
             return launch_em_cluster<kEmManyThreads, kEmManyValues>(values, windows, n_windows, ctas, out_mean, out_sd, st);
         ctas = 1;
         while ((long long)ctas * kEmClusterThreads * kEmMaxValues < max_window) ctas *= 2;
         // (a barrier of the cluster costs as much as a dozen samples per thread)
-        while (ctas < kEmMaxCluster && (long long)n_windows * ctas * 2 <= 148 &&
+        while (ctas < kEmMaxCluster && (long long)n_windows * ctas * 2 <= kEmSms &&
                (long long)ctas * kEmClusterThreads * 12 < max_window)
             ctas *= 2;
         const long long per = (max_window + (long long)ctas * kEmClusterThreads - 1) / ((long long)ctas * kEmClusterThreads);

@@ -32,6 +32,13 @@ def test_sigma_with_many_windows(gpu, port, n, zwindow):
     _check(port, (600, 17, 18), n, "z-adaptive", zwindow, False)
 
 
+@pytest.mark.parametrize("nz,n,zwindow", [(222, 88000, 100), (221, 88000, 100),  # CTAs: two waves or fewer
+                                          (300, 84000, 100), (300, 88000, 100),  # 0.7 full or less
+                                          (1000, 99000, 100)])                   # one CTA per window
+def test_sigma_at_the_edges_of_many_windows(gpu, port, nz, n, zwindow):
+    _check(port, (nz, 17, 18), n, "z-adaptive", zwindow, False)
+
+
 @pytest.mark.parametrize("n,zwindow", [(60000, 140), (100000, 400)])
 def test_more_clusters_than_the_gpu_holds(gpu, n, zwindow):
     """Hundreds of windows of two and of eight CTAs each: clusters start as others
