@@ -235,14 +235,21 @@ double plan_time(const PairArgs& a, const int* pr, int sms, const Plan& p) {
     return (dist + weights) * blocks;
 }
 
-// Whether a plan is worth running: the single-pass kernels take kSingle times as
+// Whether a plan is worth running. With few offsets the two launches and the
+// distances' way through memory cost more than the pairs save: single-pass over
+// paired time at patch radius 1, 2 offsets 0.60 to 0.68, 6 offsets 0.83 to 0.88, 8
+// offsets 0.93 to 1.08, 14 to 18 offsets 0.96 to 1.45, from 28 on at least 1.17; at
+// patch radius 2 and 3, 2 offsets 0.67 to 1.11, 4 offsets 0.89 to 1.43, from 6 on
+// 1.09 to 1.6; fused, 8 offsets 0.81 and 0.97 on 24 x 64 x 64 (five volumes of 23
+// thousand to 16.8 million voxels). And with little workspace: the single-pass kernels take kSingle times as
 // long as the whole volume in one chunk, so a plan that is cut up further is slower
 // than they are. Measured at 256^3 as workspace: paired (single-pass), ms. Patch
 // radius 1, search radius 10, 22 GB: 92.9, 16: 96.8, 8: 113.7, 4: 130.9, 2: 149, 1:
 // 296 (102.6); search radius 5, 22 GB: 13.9, 2: 16.1, 1: 20.0 (17.1). Patch radius
 // 2, search radius 5, 22 GB: 19.7, 1: 27.3, 0.5: 30.8, 0.25: 42.5 (36.1). Patch
 // radius 3, search radius 7, 22 GB: 112, 2: 138, 1: 167, 0.5: 221, 0.25: 396 (262).
-bool plan_pays(const PairArgs& a, const int* pr, int sms, int warps, const Plan& p) {
+bool plan_pays(const PairArgs& a, const int* pr, bool fused, int sms, int warps, const Plan& p) {
+    if (a.S < (pr[0] == 1 ? 14 : fused ? 10 : 6)) return false;
     const double kSingle = pr[0] == 1 ? 1.18 : pr[0] == 2 ? 1.85 : 2.3;
     return p.cost > 0 && plan_time(a, pr, sms, p) <= kSingle * plan_time(a, pr, sms, plan_blocks(a, pr, sms, warps, SIZE_MAX));
 }
@@ -289,7 +296,7 @@ int inlm::pair_plan(inlm_denoiser* d) {
     const Plan plan = plan_blocks(a, pr, r.sms, r.warps, budget);
     r.active = false;
     a.dist = nullptr;  // no tensor maps yet
-    if (plan.cost == 0 || (!r.forced && !plan_pays(a, pr, r.sms, r.warps, plan))) return INLM_OK;
+    if (plan.cost == 0 || (!r.forced && !plan_pays(a, pr, d->p.precision == INLM_PRECISION_F32_FMA, r.sms, r.warps, plan))) return INLM_OK;
     r.bx = plan.bx;
     r.by = plan.by;
     r.chunk = plan.chunk;
@@ -547,7 +554,7 @@ extern "C" int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, in
     if (!pair_extents(g, shape, p->nslices, 227 * 1024, &a)) return fail(INLM_ERR_UNSUPPORTED, "the box does not fit");
     const Plan most = plan_blocks(a, pr, 148, pair_kernel_warps(pr[0]), SIZE_MAX);
     const Plan plan = plan_blocks(a, pr, 148, pair_kernel_warps(pr[0]), (size_t)bytes);
-    const double runs = plan_pays(a, pr, 148, pair_kernel_warps(pr[0]), plan) ? 1.0 : 0.0;
+    const double runs = plan_pays(a, pr, p->precision == INLM_PRECISION_F32_FMA, 148, pair_kernel_warps(pr[0]), plan) ? 1.0 : 0.0;
     const double v[8] = {runs, plan.cost > 0 ? plan_time(a, pr, 148, plan) : 0.0, plan_time(a, pr, 148, most), (double)plan.bytes(a.H), (double)plan.bx,
                          (double)plan.by, (double)plan.chunk, (double)plan.tz};
     std::copy(v, v + 8, out);

@@ -36,6 +36,17 @@ def test_the_faster_form_is_chosen(lib, shape, pr, sr, gb, paired, single):
     assert runs == (paired < single), ratio
 
 
+@pytest.mark.parametrize("pr,sr,paired", [
+    (1, (1, 1, 1), False), (1, (0, 0, 2), False), (1, (1, 1, 2), False), (1, (2, 2, 1), True), (1, (2, 2, 2), True),
+    (2, (0, 0, 2), False), (2, (1, 1, 1), True), (3, (0, 0, 1), False), (3, (1, 1, 2), True),
+])
+def test_few_offsets_run_single_pass(lib, pr, sr, paired):
+    cp = DenoiseParameters(radius_patchspace=(pr,) * 3, radius_searchspace=sr).to_c()
+    out = (C.c_double * 8)()
+    _lib.check(lib.inlm_debug_pair_plan((C.c_int * 3)(256, 256, 256), C.byref(cp), 64 * GB, out), "pair_plan")
+    assert bool(out[0]) == paired
+
+
 def test_less_workspace_is_never_planned_as_faster(lib):
     ratios = [plan(lib, (256, 256, 256), 2, 7, gb * GB)[1] for gb in (32, 16, 8, 4, 2, 1, 0.5, 0.25)]
     assert ratios == sorted(ratios) and ratios[0] >= 1
