@@ -248,9 +248,11 @@ double plan_time(const PairArgs& a, const int* pr, int sms, const Plan& p) {
 // 296 (102.6); search radius 5, 22 GB: 13.9, 2: 16.1, 1: 20.0 (17.1). Patch radius
 // 2, search radius 5, 22 GB: 19.7, 1: 27.3, 0.5: 30.8, 0.25: 42.5 (36.1). Patch
 // radius 3, search radius 7, 22 GB: 112, 2: 138, 1: 167, 0.5: 221, 0.25: 396 (262).
-bool plan_pays(const PairArgs& a, const int* pr, bool fused, int sms, int warps, const Plan& p) {
+// Where the column form does not fit (patch radius 1, search radius 13: 174 against
+// 389 ms) the tile kernels set the line.
+bool plan_pays(const PairArgs& a, const int* pr, bool fused, bool column, int sms, int warps, const Plan& p) {
     if (a.S < (pr[0] == 1 ? 14 : fused ? 10 : 6)) return false;
-    const double kSingle = pr[0] == 1 ? 1.18 : pr[0] == 2 ? 1.85 : 2.3;
+    const double kSingle = column ? 1.18 : pr[0] <= 2 ? 1.85 : 2.3;
     return p.cost > 0 && plan_time(a, pr, sms, p) <= kSingle * plan_time(a, pr, sms, plan_blocks(a, pr, sms, warps, SIZE_MAX));
 }
 
@@ -296,7 +298,8 @@ int inlm::pair_plan(inlm_denoiser* d) {
     const Plan plan = plan_blocks(a, pr, r.sms, r.warps, budget);
     r.active = false;
     a.dist = nullptr;  // no tensor maps yet
-    if (plan.cost == 0 || (!r.forced && !plan_pays(a, pr, d->p.precision == INLM_PRECISION_F32_FMA, r.sms, r.warps, plan))) return INLM_OK;
+    const bool fused = d->p.precision == INLM_PRECISION_F32_FMA;
+    if (plan.cost == 0 || (!r.forced && !plan_pays(a, pr, fused, d->tcfg.column, r.sms, r.warps, plan))) return INLM_OK;
     r.bx = plan.bx;
     r.by = plan.by;
     r.chunk = plan.chunk;
@@ -552,12 +555,24 @@ extern "C" int inlm_debug_pair_plan(const int shape[3], const inlm_params* p, in
     const Geometry g = make_geometry(p->search_radius, pr, p->nslices, p->z_anisotropy, p->weight_table, shape[2] + 2 * pz);
     PairArgs a;
     if (!pair_extents(g, shape, p->nslices, 227 * 1024, &a)) return fail(INLM_ERR_UNSUPPORTED, "the box does not fit");
-    const Plan most = plan_blocks(a, pr, 148, pair_kernel_warps(pr[0]), SIZE_MAX);
-    const Plan plan = plan_blocks(a, pr, 148, pair_kernel_warps(pr[0]), (size_t)bytes);
-    const double runs = plan_pays(a, pr, p->precision == INLM_PRECISION_F32_FMA, 148, pair_kernel_warps(pr[0]), plan) ? 1.0 : 0.0;
-    const double v[8] = {runs, plan.cost > 0 ? plan_time(a, pr, 148, plan) : 0.0, plan_time(a, pr, 148, most), (double)plan.bytes(a.H), (double)plan.bx,
-                         (double)plan.by, (double)plan.chunk, (double)plan.tz};
-    std::copy(v, v + 8, out);
+    const int sms = 148, warps = pair_kernel_warps(pr[0]);
+    const Plan most = plan_blocks(a, pr, sms, warps, SIZE_MAX);
+    const Plan plan = plan_blocks(a, pr, sms, warps, (size_t)bytes);
+    TileArgs t{};
+    const int depth = column_kernel_depth(pr[0], pr[1], pr[2]);
+    t.pbx = (32 + 2 * a.px + 3) / 4 * 4;
+    t.pby = 8 + 2 * a.py;
+    t.pbz = depth + 2 * a.pz;
+    const bool column = depth > 0 && column_smem_bytes(t) <= 227 * 1024;
+    const bool runs = plan_pays(a, pr, p->precision == INLM_PRECISION_F32_FMA, column, sms, warps, plan);
+    out[0] = runs ? 1.0 : 0.0;
+    out[1] = plan.cost > 0 ? plan_time(a, pr, sms, plan) : 0.0;
+    out[2] = plan_time(a, pr, sms, most);
+    out[3] = (double)plan.bytes(a.H);
+    out[4] = plan.bx;
+    out[5] = plan.by;
+    out[6] = plan.chunk;
+    out[7] = plan.tz;
     return INLM_OK;
 }
 

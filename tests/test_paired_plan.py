@@ -28,6 +28,7 @@ def plan(lib, shape, pr, sr, size):
     ((256, 256, 256), 2, 5, 0.25, 42.45, 36.15), ((256, 256, 256), 2, 7, 2, 70.1, 105.3),
     ((256, 256, 256), 2, 7, 0.25, 249.7, 105.3), ((256, 256, 256), 3, 7, 2, 137.5, 261.7),
     ((256, 256, 256), 3, 7, 0.25, 395.9, 261.7), ((512, 512, 512), 3, 7, 2, 1118.8, 2073.3),
+    ((256, 256, 256), 1, 13, 8, 224.4, 389.0),  # (the column form does not fit)
     ((61, 187, 203), 3, 7, 1, 23.8, 46.5), ((61, 187, 203), 3, 7, 0.25, 82.2, 46.5),
 ])
 def test_the_faster_form_is_chosen(lib, shape, pr, sr, gb, paired, single):
