@@ -164,7 +164,7 @@ def measured_peaks():
 # traffic grows with the volume (its halo share is a little smaller at 512^3).
 FILTER_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, one 256x256x96 pass of "
                          "nlm_pair_dist_kernel and nlm_pair_weight_kernel, scaled by the voxels")
-FILTER_TRAFFIC_BYTES_PER_LAUNCH = (512.0 ** 3 / (256 * 256 * 96)) * (7.796173e9 + 13.552841e9)
+FILTER_TRAFFIC_BYTES_PER_LAUNCH = (512.0 ** 3 / (256 * 256 * 96)) * (7.797787e9 + 13.568617e9)
 
 
 def fp32_arithmetic_peak(device: int):

@@ -355,10 +355,11 @@ int inlm_net_input(inlm_denoiser* d, float* vol_dev, float* scale_dev);
  * kernel configuration per run (main.cpp:311-545). */
 
 /* Restricts the plain FP32 filter to one kernel family and picks its first
- * configuration that fits: form 0 = automatic (the column form for patch
- * radius 1 when it fits; the warp-specialised kernel where patch sums
- * dominate, at 100 or more patch taps or at 30 or more taps with 400 or more
- * search offsets; else the tiled kernels), 1 = the tiled kernels without warp
+ * configuration that fits: form 0 = automatic (the paired form where it is the
+ * faster one; in a single pass the column form for patch radius 1 when it fits;
+ * the warp-specialised kernel where patch sums dominate, at 100 or more patch
+ * taps or at 30 or more taps with 400 or more search offsets; else the tiled
+ * kernels), 1 = the tiled kernels without warp
  * specialisation, 2 = the column form only, 3 = the warp-specialised kernel
  * only (INLM_ERR_UNSUPPORTED where the form has no instantiation or does not
  * fit). Results do not change: every form rounds each voxel identically. Call
@@ -381,9 +382,9 @@ typedef struct inlm_batch inlm_batch;
 
 /* n volumes of different sizes and radii filtered together: shapes holds
  * {nx, ny, nz} per volume, params one inlm_params per volume (plain FP32,
- * noise mode global, z-adaptive or manual, one device). Each iteration of all
- * volumes runs as one persistent kernel over their tiles (heaviest tiles
- * first; tile configurations from the autotuner; volumes whose patch shape has
+ * noise mode global, z-adaptive or manual, one device). Each iteration of the
+ * small volumes runs as one persistent kernel over their tiles, volumes of a tile
+ * per SM or more run the paired form one after another (heaviest tiles first; tile configurations from the autotuner; volumes whose patch shape has
  * no batched body get their own launch), and the whole schedule (noise
  * estimates, padding, iterations) is captured once in a CUDA graph. At most 24
  * batched volumes. */

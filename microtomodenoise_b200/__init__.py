@@ -220,7 +220,8 @@ class IterativeNLM_GPU:
         return buf.value.decode()
 
     def select_tile_form(self, form: str = "auto") -> str:
-        """Plain FP32 kernel family: "auto", "tile" (the tiled kernels without
+        """Plain FP32 kernel family: "auto" (the paired form where it is the
+        faster one, else the best single-pass kernel), "tile" (the tiled kernels without
         warp specialisation), "column" (the column form, patch radius 1) or
         "ws" (the warp-specialised kernel). Results do not change; returns
         describe()."""

@@ -768,11 +768,11 @@ int inlm::tile_config_try(inlm_denoiser* d, int tz, bool raw_smem, bool* ok, boo
 }
 
 // The single-pass kernel (before any autotuning): the first candidate that
-// fits. It runs where the paired form (api_pair.cu) does not: no workspace, a
-// form selected by name, small volumes of a batch, the fused form at patch radius
-// 1 on volumes that fill the SMs. Everywhere else the paired form is faster,
-// measured over patch shapes, search radii 2 to 10 and 36 volumes of 27 thousand
-// to 18 million voxels: 1.02 to 1.4 times at patch radius 1, 1.7 to 2.7 times at
+// fits. It runs where the paired form (api_pair.cu) does not: few search offsets,
+// too little room for its workspace, a form selected by name, small volumes of a
+// batch, the fused form at patch radius 1 on volumes that fill the SMs.
+// Everywhere else the paired form is faster, measured over eight patch shapes:
+// from search radius 2 on 1.05 to 1.9 times at patch radius 1, 1.2 to 3.7 times at
 // radius 2 and 3, more where few tiles leave SMs idle.
 // form: 0 every candidate, 1 the tiled kernels only, 2 the column form only,
 // 3 the warp-specialised kernel only. In form 0 the warp-specialised kernel
