@@ -294,12 +294,14 @@ int inlm::pair_plan(inlm_denoiser* d) {
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
     size_t budget = std::min(total_b / kWorkspaceShare, (free_b + idle_bytes(d->device)) / 2);
     if (r.limit > 0) budget = std::min(budget, r.limit);
-    a.tz = r.tz;
-    const Plan plan = plan_blocks(a, pr, r.sms, r.warps, budget);
+    PairArgs deepest = a;  // (without a new plan the old one stays whole)
+    deepest.tz = r.tz;
+    const Plan plan = plan_blocks(deepest, pr, r.sms, r.warps, budget);
     r.active = false;
-    a.dist = nullptr;  // no tensor maps yet
     const bool fused = d->p.precision == INLM_PRECISION_F32_FMA;
-    if (plan.cost == 0 || (!r.forced && !plan_pays(a, pr, fused, d->tcfg.column, r.sms, r.warps, plan))) return INLM_OK;
+    if (plan.cost == 0 || (!r.forced && !plan_pays(deepest, pr, fused, d->tcfg.column, r.sms, r.warps, plan)))
+        return INLM_OK;
+    a.dist = nullptr;  // no tensor maps yet
     r.bx = plan.bx;
     r.by = plan.by;
     r.chunk = plan.chunk;

@@ -192,6 +192,37 @@ def test_first_pass_allocates_its_workspace_and_nothing_else(gpu, port):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("pr,sr,form", [((1, 1, 1), (5, 5, 5), "column"), ((2, 2, 2), (4, 4, 4), None)])
+def test_memory_gets_scarce_and_free_again(gpu, pr, sr, form):
+    """Somebody else takes the memory between configuration and a pass: the passes
+    are planned anew for what is left, or run single-pass where that plan would be
+    slower; with the memory back, the handle's plan is whole."""
+    torch = pytest.importorskip("torch")
+    raw = synth.small_case((64, 128, 128), seed=8)
+    sig = _sigmas(64)[1]
+    g = IterativeNLM_GPU()
+    g.configure_device(raw.shape, DenoiseParameters(radius_patchspace=pr, radius_searchspace=sr))
+    g.set_sigma(sig)
+    assert "paired" in g.describe()
+    g.Run_GaussianNoise(1, raw)
+    want = g.get_result()
+    trim_memory()
+    free = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(free - (600 << 20), dtype=torch.uint8, device="cuda")
+    g.Run_GaussianNoise(1, raw)
+    assert np.array_equal(g.get_result(), want)
+    del hog
+    torch.cuda.empty_cache()
+    g.Run_GaussianNoise(1, raw)
+    assert np.array_equal(g.get_result(), want)
+    if form:
+        g.select_tile_form(form)
+        g.Run_GaussianNoise(1, raw)
+        assert np.array_equal(g.get_result(), want)
+    g.free_device()
+
+
+@pytest.mark.gpu
 def test_paired_handles_take_turns_on_one_workspace(gpu):
     L = _lib.load()
     live = C.c_int64(0)
