@@ -36,9 +36,11 @@ Pool g_pool[kMaxDevices];
 std::recursive_mutex g_pool_mutex;  // device_malloc may call pair_trim under it
 std::atomic<long long> g_pool_bound{0};  // a test's bound in place of the share
 
+// (a batch's own does not count: it would leave the calls beside it nothing)
 size_t pool_bytes(const Pool& pool) {
     size_t n = 0;
-    for (const PairBuf* b : pool.bufs) n += b->bytes;
+    for (const PairBuf* b : pool.bufs)
+        if (!b->alone) n += b->bytes;
     return n;
 }
 
@@ -104,6 +106,7 @@ void hand_back(PairBuf* b) {
     Pool& pool = g_pool[b->device];
     if (--b->users > 0) return;
     b->last = nullptr;
+    b->alone = false;
     while ((pool.users == 0 || pool_bytes(pool) > pool_share(pool)) && free_idle(pool)) {
     }
 }

@@ -7,7 +7,7 @@ import threading
 import numpy as np
 import pytest
 
-from microtomodenoise_b200 import DenoiseParameters, IterativeNLM_GPU, _lib, synth, trim_memory
+from microtomodenoise_b200 import Batch, DenoiseParameters, IterativeNLM_GPU, _lib, synth, trim_memory
 from oracle.oracle import FilterParams
 
 MB = 1 << 20
@@ -335,6 +335,34 @@ def test_threads_share_workspaces(gpu, bound):
     for g in handles:
         g.free_device()
     assert live() == before
+
+
+@pytest.mark.gpu
+def test_a_batch_beside_a_handle_leaves_the_pool_its_share(gpu):
+    L = _lib.load()
+
+    def live():
+        n = C.c_int64(0)
+        _lib.check(L.inlm_debug_live_allocations(C.byref(n)), "live allocations")
+        return n.value
+
+    raw = synth.small_case((20, 24, 40), seed=5)
+    g = IterativeNLM_GPU()
+    g.configure_device(raw.shape, DenoiseParameters(radius_patchspace=(2, 2, 2), radius_searchspace=(3, 3, 3)))
+    g.set_sigma(_sigmas(20)[1])
+    _lib.check(L.inlm_debug_pair_pool(32 * MB), "pair_pool")  # the handle's takes 11, the batch's more than 32
+    try:
+        b = Batch([(32, 64, 160)], [DenoiseParameters(radius_patchspace=(1, 1, 1), radius_searchspace=(4, 4, 4),
+                                                      noise_mode="manual", sigma=(0.06, 0.05))])
+        assert "own launch paired" in b.describe(), b.describe()
+        before = live()
+        for _ in range(2):
+            g.Run_GaussianNoise(1, raw)
+            assert live() == before + 1  # kept for the next call
+        b.close()
+    finally:
+        L.inlm_debug_pair_pool(0)
+    g.free_device()
 
 
 @pytest.mark.gpu
